@@ -31,6 +31,7 @@
 #include "rsv_gate.h"
 #include "rsv_device.cuh"
 #include "rsv_launch.h"
+#include "rsv_ring.h"
 #include "rsv_tma.h"
 #include "rsv_types.h"
 
@@ -891,6 +892,13 @@ struct rsv_backend {
   // coset tables, per-tile Z, coset sums, per-CTA G/F and their sums
   rsv::DevBuf<double2> mps_tsite, mps_btab, mps_coslo, mps_coshi, mps_mtab, mps_wtab, mps_zt, mps_ylo, mps_yhi, mps_partials,
       mps_gf;
+  // contraction along the ring (rsv_ring.cu) instead of the tile passes, its
+  // kept components, energy shares and counter, and the field of the last forward
+  bool ring = false;
+  double ring_field = 0.0;
+  rsv::DevBuf<double2> ring_left, ring_right;
+  rsv::DevBuf<double> ring_energy;
+  rsv::DevBuf<unsigned int> ring_counter;
   rsv::DevBuf<int> tables;  // pass_grid | theta_pass | theta_slot | phi_pass
   rsv::DevBuf<int> order;   // undo order of the wires within a backward layer
   rsv::DevBuf<double2> rot;
@@ -1243,6 +1251,81 @@ void launch_prep(rsv_backend *B, cudaStream_t st) {
   }
 }
 
+// Which circuits are contracted along the ring: the cost there is n 16^(L-1) L
+// against 2^n n L on the tile passes.  Up to 4 layers it is the faster one from
+// the smallest circuit on (n = 3, L = 1: 22 us against 41; n = 12, L = 4: 30
+// against 138); 5 layers cross between n = 20 (410 us against 322) and n = 22
+// (427 against 807).
+bool ring_rule(int n, int L) { return n >= 3 && (L <= 4 || (L == 5 && n >= 21)); }
+
+// Switch a backend to the ring contraction where the rule takes it; without
+// memory for its components the tile passes stay.
+void setup_ring(rsv_backend *B) {
+  B->ring = false;
+  if (!ring_rule(B->n, B->L)) return;
+  const size_t chains = static_cast<size_t>(ring_chains(B->L)), values = ring_component_values(B->n, B->L);
+  try {
+    if (B->ring_left.count < values) B->ring_left.alloc(values);
+    if (B->ring_right.count < values) B->ring_right.alloc(values);
+    if (B->ring_energy.count < chains + 1) B->ring_energy.alloc(chains + 1);
+    if (B->ring_counter.p == nullptr) {
+      B->ring_counter.alloc(1);
+      check(cudaMemset(B->ring_counter.p, 0, sizeof(unsigned int)), "ring counter clear");
+    }
+  } catch (const Error &e) {
+    if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
+    cudaGetLastError();  // clear the allocation failure
+    return;
+  }
+  B->ring = true;
+}
+
+void leave_ring(rsv_backend *B) {
+  B->ring = false;
+  B->ring_left.release();
+  B->ring_right.release();
+}
+
+// A caller that chose a backward schedule, fewer analytic layers or other
+// kernels chose a tile-pass plan; the defaults choose by the rule.
+void refresh_ring(rsv_backend *B) {
+  const bool defaults = B->backward_mode == RSV_BACKWARD_AUTO && B->analytic_layers == kDefaultAnalyticLayers &&
+                        B->kernel_flags == (RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY) && B->force_c == 0;
+  if (defaults && !B->dense && !B->gate_level) setup_ring(B);
+  else leave_ring(B);
+}
+
+RingParams ring_params(rsv_backend *B, double *energy_out, double *grad_out) {
+  RingParams R{};
+  R.n = B->n;
+  R.L = B->L;
+  R.field = B->ring_field;
+  R.coef = B->coef.p;
+  R.left = B->ring_left.p;
+  R.right = B->ring_right.p;
+  R.energy_parts = B->ring_energy.p;
+  R.counter = B->ring_counter.p;
+  R.energy_out = energy_out;
+  R.grad_out = grad_out;
+  return R;
+}
+
+// keep: the left components stay for a later run_ring_backward
+void run_ring(rsv_backend *B, bool grad, bool keep, double *energy_out, double *grad_out, cudaStream_t st) {
+  B->ring_field = B->field;
+  const RingParams R = ring_params(B, energy_out, grad_out);
+  timed(B, st, 1, 0.0, [&] { check(launch_ring_sweeps(R, true, grad, grad || keep, st), "ring sweep launch"); });
+  if (grad) timed(B, st, 3, 0.0, [&] { check(launch_ring_gradient(R, st), "ring gradient launch"); });
+}
+
+void run_ring_backward(rsv_backend *B, double *grad_out, cudaStream_t st) {
+  const RingParams R = ring_params(B, nullptr, grad_out);
+  timed(B, st, 3, 0.0, [&] {
+    check(launch_ring_sweeps(R, false, true, false, st), "ring sweep launch");
+    check(launch_ring_gradient(R, st), "ring gradient launch");
+  }, 2);
+}
+
 // Gate-level path: RY, RZ and CNOT as separate kernels and the inverse walk
 // (the reference's inverse_walk_cuQuantum schedule without cuStateVec).
 void run_gate_level(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cudaStream_t st) {
@@ -1261,7 +1344,8 @@ void run_gate_level(rsv_backend *B, bool grad, double *energy_out, double *grad_
   check(rsv::run_gate_level(A, st), "gate-level launch");
 }
 
-void run_all(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cudaStream_t st) {
+// keep: an energy-only call whose gradient may be asked for later
+void run_all(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cudaStream_t st, bool keep = false) {
   ++B->generation;
   B->forward_only_state = false;
   if (B->gate_level) {
@@ -1278,6 +1362,10 @@ void run_all(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cu
     D.energy_out = energy_out;
     D.grad_out = grad ? grad_out : nullptr;
     check(run_dense_scan(D, st), "dense_scan launch");
+    return;
+  }
+  if (B->ring) {
+    run_ring(B, grad, keep, energy_out, grad_out, st);
     return;
   }
   launch_prep(B, st);
@@ -1882,6 +1970,7 @@ void setup_plan(rsv_backend *B, int mode) {
 struct TuneChoice {
   int mode = RSV_BACKWARD_AUTO, analytic = kDefaultAnalyticLayers;
   int kernels = RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY, force_c = 0;
+  bool ring = false;  // contraction along the ring instead of a tile-pass plan
   double ms = 0.0;
 };
 
@@ -1900,9 +1989,12 @@ void apply_choice(rsv_backend *B, const TuneChoice &c) {
   B->kernel_flags = c.kernels;
   B->force_c = c.force_c;
   setup_plan(B, c.mode);
+  if (c.ring) setup_ring(B);
+  else leave_ring(B);
 }
 
 std::string choice_str(const rsv_backend *B, const TuneChoice &c) {
+  if (c.ring) return "ring contraction";
   std::ostringstream os;
   os << "mode=" << (B->plan.checkpoint ? "checkpoint" : "uncompute") << " analytic_layers=" << c.analytic
      << " tma=" << ((c.kernels & RSV_KERNELS_TMA) ? 1 : 0) << " tma_passes=" << B->tma_passes
@@ -1933,12 +2025,18 @@ double time_plan(rsv_backend *B, const double *d_params, int repeats, cudaStream
   return static_cast<double>(ms) / repeats;
 }
 
-// The candidates: both backward schedules (checkpoint only where it fits),
+// The candidates: the ring contraction where the rule takes it, then the
+// tile-pass plans: both backward schedules (checkpoint only where it fits),
 // three or two analytic leading layers, the TMA kernels on (with or without
 // the fused energy) or off, and every
 // contiguous run length c of the high tiles that gives the fewest passes.
 std::vector<TuneChoice> tune_candidates(const rsv_backend *B) {
   std::vector<TuneChoice> out;
+  if (ring_rule(B->n, B->L)) {
+    TuneChoice t;
+    t.ring = true;
+    out.push_back(t);
+  }
   std::vector<int> cs = {0};
   if (B->n > 12) {
     auto passes = [&](int c) { return static_cast<int>(high_tiles(B->n, 12, 2, c).size()); };
@@ -2059,6 +2157,7 @@ rsv_status rsv_create(int num_qubits, int num_layers, double field, const char *
       B->gate_grid = gate_grid(num_qubits, B->sms);
       B->gate_partials.alloc(static_cast<size_t>(B->gate_grid) * (1 + 2 * nl));
     }
+    refresh_ring(B.get());
     B->coef.alloc(nl);
     B->ptab.alloc(static_cast<size_t>(num_layers) * 1024);
     B->outputs.alloc(1 + B->num_params);
@@ -2133,7 +2232,7 @@ rsv_status rsv_forward_device(rsv_backend *B, const double *d_params, size_t num
     if (d_energy_out == nullptr) invalid("d_energy_out is null");
     cudaStream_t st = device_stream(stream);
     check(launch_coef(d_params, B->coef.p, static_cast<int>(B->n * B->L), st), "coef launch");
-    run_all(B, false, d_energy_out, nullptr, st);
+    run_all(B, false, d_energy_out, nullptr, st, true);
     B->forward_only_state = true;
     if (generation_out) *generation_out = B->generation;
   });
@@ -2149,9 +2248,13 @@ rsv_status rsv_backward_device(rsv_backend *B, unsigned long long generation,
       throw Error(RSV_ERR_STALE_STATE,
                   "backward needs the state of the matching forward; the backend ran another call since");
     cudaStream_t st = device_stream(stream);
-    run_backward(B, st, false);  // the forward call computed the whole energy
-    // energy is rewritten with the same value into the outputs scratch slot
-    run_finalize(B, true, B->outputs.p, d_gradient_out, st);
+    if (B->ring) {
+      run_ring_backward(B, d_gradient_out, st);
+    } else {
+      run_backward(B, st, false);  // the forward call computed the whole energy
+      // energy is rewritten with the same value into the outputs scratch slot
+      run_finalize(B, true, B->outputs.p, d_gradient_out, st);
+    }
     B->forward_only_state = false;
     ++B->generation;
   });
@@ -2185,6 +2288,16 @@ rsv_status rsv_profile_energy_and_grad(rsv_backend *B, const double *params, siz
       run_all(B, grad, B->outputs.p, B->outputs.p + 1, st);
       cudaEventRecord(ev[2], st);
       cudaEventRecord(ev[3], st);
+      cudaEventRecord(ev[4], st);
+    } else if (B->ring) {
+      // the sweeps (energy included) as the forward stage, the gradient as the backward
+      B->ring_field = B->field;
+      const RingParams R = ring_params(B, B->outputs.p, B->outputs.p + 1);
+      cudaEventRecord(ev[1], st);
+      check(launch_ring_sweeps(R, true, grad, grad, st), "ring sweep launch");
+      cudaEventRecord(ev[2], st);
+      cudaEventRecord(ev[3], st);
+      if (grad) check(launch_ring_gradient(R, st), "ring gradient launch");
       cudaEventRecord(ev[4], st);
     } else {
       launch_prep(B, st);
@@ -2313,6 +2426,7 @@ rsv_status rsv_set_backward_mode(rsv_backend *B, int mode) {
     if (B == nullptr) invalid("backend is null");
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     setup_plan(B, mode);
+    refresh_ring(B);
   });
 }
 
@@ -2324,6 +2438,7 @@ rsv_status rsv_set_analytic_layers(rsv_backend *B, int max_layers) {
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     B->analytic_layers = max_layers;
     setup_plan(B, B->backward_mode);
+    refresh_ring(B);
   });
 }
 
@@ -2335,6 +2450,7 @@ rsv_status rsv_set_kernels(rsv_backend *B, int flags) {
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     B->kernel_flags = flags;
     setup_plan(B, B->backward_mode);
+    refresh_ring(B);
   });
 }
 
@@ -2368,7 +2484,7 @@ rsv_status rsv_autotune(rsv_backend *B, const double *d_params, size_t num_param
       }
     }
     std::ostringstream rep;
-    const TuneChoice before{B->backward_mode, B->analytic_layers, B->kernel_flags, B->force_c, 0.0};
+    const TuneChoice before{B->backward_mode, B->analytic_layers, B->kernel_flags, B->force_c, B->ring, 0.0};
     TuneChoice best;
     best.ms = 1e300;
     std::vector<std::string> seen;
@@ -2386,7 +2502,7 @@ rsv_status rsv_autotune(rsv_backend *B, const double *d_params, size_t num_param
         continue;
       }
       // the same launches under another name are timed once
-      std::string sig = describe(B->plan) + " fused_energy=" + std::to_string(B->energy_fuse_pass) +
+      std::string sig = std::string(B->ring ? "ring " : "") + describe(B->plan) + " fused_energy=" + std::to_string(B->energy_fuse_pass) +
                         std::to_string(B->energy_defer_pass);
       if (std::find(seen.begin(), seen.end(), sig) != seen.end()) continue;
       seen.push_back(sig);
@@ -2421,6 +2537,7 @@ rsv_status rsv_describe_backend(rsv_backend *B, char *buf, size_t buf_size, size
     os << "analytic_layers=" << B->analytic_layers << " kernels=" << B->kernel_flags
        << " high_tile_c=" << (B->force_c ? std::to_string(B->force_c) : std::string("planner"))
        << " tma_passes=" << B->tma_passes;
+    if (B->ring) os << " ring_contraction (the plan below is not used)";
     if (B->energy_fuse_pass >= 0)
       os << " fused_energy: backward pass " << B->energy_fuse_pass << " applies "
          << kTmaNumEnergyMasks << " field terms,"
