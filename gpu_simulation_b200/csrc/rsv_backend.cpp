@@ -27,6 +27,7 @@
 
 #include "../../include/rsv.h"
 #include "rsv_batch.h"
+#include "rsv_cluster.h"
 #include "rsv_dense.h"
 #include "rsv_gate.h"
 #include "rsv_device.cuh"
@@ -847,6 +848,10 @@ const char *kStageNames[kNumStages] = {
 }  // namespace
 }  // namespace rsv
 
+namespace rsv {
+enum class Path { kPasses, kRing, kCluster };
+}
+
 struct rsv_backend {
   int n = 0, L = 0;
   double field = 0.0;
@@ -874,7 +879,7 @@ struct rsv_backend {
   int force_c = 0;  // contiguous low bits of the high tiles (0: the planner's choice)
   std::string tune_report;  // the last rsv_autotune's candidates and choice
   std::vector<rsv::TmaPass> tma;    // per backward step (used where step.kernel is kKernelTma)
-  rsv::DevBuf<int> pipeline_err;    // set by a TMA pass whose pipeline wait gave up
+  rsv::DevBuf<int> pipeline_err;    // set by a TMA pass whose pipeline wait gave up; then the ring kernels' counters
   int tma_passes = 0;
   int analytic_layers = 3;  // rsv_set_analytic_layers (default: layers 0..2 as a matrix-product state)
   // gradient_strategy "inverse_walk_cuQuantum": gate-level kernels (rsv_gate.cu)
@@ -892,13 +897,12 @@ struct rsv_backend {
   // coset tables, per-tile Z, coset sums, per-CTA G/F and their sums
   rsv::DevBuf<double2> mps_tsite, mps_btab, mps_coslo, mps_coshi, mps_mtab, mps_wtab, mps_zt, mps_ylo, mps_yhi, mps_partials,
       mps_gf;
-  // contraction along the ring (rsv_ring.cu) instead of the tile passes, its
-  // kept components, energy shares and counter, and the field of the last forward
-  bool ring = false;
-  double ring_field = 0.0;
-  rsv::DevBuf<double2> ring_left, ring_right;
-  rsv::DevBuf<double> ring_energy;
-  rsv::DevBuf<unsigned int> ring_counter;
+  // what runs a call: the tile passes, the contraction along the ring
+  // (rsv_ring.cu; its kept components lie in the state buffers) or the
+  // cluster-resident state (rsv_cluster.cu); and the field of the last forward
+  rsv::Path path = rsv::Path::kPasses;
+  rsv::ClusterShape cluster_shape{0, 4};
+  double forward_field = 0.0;
   rsv::DevBuf<int> tables;  // pass_grid | theta_pass | theta_slot | phi_pass
   rsv::DevBuf<int> order;   // undo order of the wires within a backward layer
   rsv::DevBuf<double2> rot;
@@ -1251,79 +1255,74 @@ void launch_prep(rsv_backend *B, cudaStream_t st) {
   }
 }
 
-// Which circuits are contracted along the ring: the cost there is n 16^(L-1) L
-// against 2^n n L on the tile passes.  Up to 4 layers it is the faster one from
-// the smallest circuit on (n = 3, L = 1: 22 us against 41; n = 12, L = 4: 30
-// against 138); 5 layers cross between n = 20 (410 us against 322) and n = 22
-// (427 against 807).
-bool ring_rule(int n, int L) { return n >= 3 && (L <= 4 || (L == 5 && n >= 21)); }
-
-// Switch a backend to the ring contraction where the rule takes it; without
-// memory for its components the tile passes stay.
-void setup_ring(rsv_backend *B) {
-  B->ring = false;
-  if (!ring_rule(B->n, B->L)) return;
-  const size_t chains = static_cast<size_t>(ring_chains(B->L)), values = ring_component_values(B->n, B->L);
-  try {
-    if (B->ring_left.count < values) B->ring_left.alloc(values);
-    if (B->ring_right.count < values) B->ring_right.alloc(values);
-    if (B->ring_energy.count < chains + 1) B->ring_energy.alloc(chains + 1);
-    if (B->ring_counter.p == nullptr) {
-      B->ring_counter.alloc(1);
-      check(cudaMemset(B->ring_counter.p, 0, sizeof(unsigned int)), "ring counter clear");
-    }
-  } catch (const Error &e) {
-    if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
-    cudaGetLastError();  // clear the allocation failure
-    return;
-  }
-  B->ring = true;
-}
-
-void leave_ring(rsv_backend *B) {
-  B->ring = false;
-  B->ring_left.release();
-  B->ring_right.release();
-}
-
-// A caller that chose a backward schedule, fewer analytic layers or other
-// kernels chose a tile-pass plan; the defaults choose by the rule.
-void refresh_ring(rsv_backend *B) {
-  const bool defaults = B->backward_mode == RSV_BACKWARD_AUTO && B->analytic_layers == kDefaultAnalyticLayers &&
-                        B->kernel_flags == (RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY) && B->force_c == 0;
-  if (defaults && !B->dense && !B->gate_level) setup_ring(B);
-  else leave_ring(B);
-}
-
-RingParams ring_params(rsv_backend *B, double *energy_out, double *grad_out) {
+RingParams ring_params(rsv_backend *B, const double *d_params, double *energy_out, double *grad_out) {
   RingParams R{};
   R.n = B->n;
   R.L = B->L;
-  R.field = B->ring_field;
+  R.field = B->forward_field;
+  R.params = d_params;
   R.coef = B->coef.p;
-  R.left = B->ring_left.p;
-  R.right = B->ring_right.p;
-  R.energy_parts = B->ring_energy.p;
-  R.counter = B->ring_counter.p;
+  R.left = B->states.p;
+  R.right = B->states.p + ring_component_values(B->n, B->L);
+  R.energy_parts = B->energy_partials.p;
+  R.grad_parts = reinterpret_cast<double *>(R.right + ring_component_values(B->n, B->L));
+  R.counter = reinterpret_cast<unsigned int *>(B->pipeline_err.p + 1);
   R.energy_out = energy_out;
   R.grad_out = grad_out;
   return R;
 }
 
-// keep: the left components stay for a later run_ring_backward
-void run_ring(rsv_backend *B, bool grad, bool keep, double *energy_out, double *grad_out, cudaStream_t st) {
-  B->ring_field = B->field;
-  const RingParams R = ring_params(B, energy_out, grad_out);
-  timed(B, st, 1, 0.0, [&] { check(launch_ring_sweeps(R, true, grad, grad || keep, st), "ring sweep launch"); });
-  if (grad) timed(B, st, 3, 0.0, [&] { check(launch_ring_gradient(R, st), "ring gradient launch"); });
+ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_out, double *grad_out) {
+  ClusterArgs A{};
+  A.n = B->n;
+  A.log_ctas = B->cluster_shape.log_ctas;
+  A.register_bits = B->cluster_shape.register_bits;
+  A.count = 1;
+  A.item.L = A.max_layers = B->L;
+  A.item.h = B->forward_field;
+  A.params = d_params;
+  A.coef = B->coef.p;
+  A.energy_out = energy_out;
+  A.grad_out = grad_out;
+  return A;
 }
 
-void run_ring_backward(rsv_backend *B, double *grad_out, cudaStream_t st) {
-  const RingParams R = ring_params(B, nullptr, grad_out);
-  timed(B, st, 3, 0.0, [&] {
-    check(launch_ring_sweeps(R, false, true, false, st), "ring sweep launch");
-    check(launch_ring_gradient(R, st), "ring gradient launch");
-  }, 2);
+// A call on the ring or the cluster path.  d_params: the angles, or null when
+// B->coef holds their cosines and sines.  keep: what a later gradient needs
+// stays (the left components, or psi and H psi; B->coef).
+void run_direct(rsv_backend *B, const double *d_params, bool grad, bool keep, double *energy_out, double *grad_out,
+                cudaStream_t st) {
+  B->forward_field = B->field;
+  if (B->path == Path::kRing) {
+    const RingParams R = ring_params(B, d_params, energy_out, grad_out);
+    timed(B, st, 1, 0.0, [&] { check(launch_ring_sweeps(R, true, grad, grad || keep, st), "ring sweep launch"); });
+    if (grad) timed(B, st, 3, 0.0, [&] { check(launch_ring_gradient(R, st), "ring gradient launch"); });
+    return;
+  }
+  ClusterArgs A = cluster_args(B, d_params, energy_out, grad ? grad_out : nullptr);
+  if (keep) {
+    A.psi = state_buf(B, 0);
+    A.lam = state_buf(B, 1);
+    A.coef_out = d_params ? B->coef.p : nullptr;
+  }
+  timed(B, st, 1, 0.0, [&] { check(launch_cluster(A, st), "cluster launch"); });
+}
+
+// The gradient of the last run_direct that kept its state.
+void run_direct_backward(rsv_backend *B, double *grad_out, cudaStream_t st) {
+  if (B->path == Path::kRing) {
+    const RingParams R = ring_params(B, nullptr, nullptr, grad_out);
+    timed(B, st, 3, 0.0, [&] {
+      check(launch_ring_sweeps(R, false, true, false, st), "ring sweep launch");
+      check(launch_ring_gradient(R, st), "ring gradient launch");
+    }, 2);
+    return;
+  }
+  ClusterArgs A = cluster_args(B, nullptr, nullptr, grad_out);
+  A.psi = state_buf(B, 0);
+  A.lam = state_buf(B, 1);
+  A.resume = 1;
+  timed(B, st, 3, 0.0, [&] { check(launch_cluster(A, st), "cluster launch"); });
 }
 
 // Gate-level path: RY, RZ and CNOT as separate kernels and the inverse walk
@@ -1344,10 +1343,21 @@ void run_gate_level(rsv_backend *B, bool grad, double *energy_out, double *grad_
   check(rsv::run_gate_level(A, st), "gate-level launch");
 }
 
-// keep: an energy-only call whose gradient may be asked for later
-void run_all(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cudaStream_t st, bool keep = false) {
+// d_params: the angles on the device, or null when B->coef holds their cosines
+// and sines.  keep: an energy-only call whose gradient may be asked for later.
+void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_out, double *grad_out,
+             cudaStream_t st, bool keep = false) {
   ++B->generation;
   B->forward_only_state = false;
+  if (B->path != Path::kPasses) {
+    run_direct(B, d_params, grad, keep, energy_out, grad_out, st);
+    return;
+  }
+  if (d_params) {
+    timed(B, st, 0, 0.0, [&] {
+      check(launch_coef(d_params, B->coef.p, static_cast<int>(B->n * B->L), st), "coef launch");
+    });
+  }
   if (B->gate_level) {
     run_gate_level(B, grad, energy_out, grad_out, st);
     return;
@@ -1362,10 +1372,6 @@ void run_all(rsv_backend *B, bool grad, double *energy_out, double *grad_out, cu
     D.energy_out = energy_out;
     D.grad_out = grad ? grad_out : nullptr;
     check(run_dense_scan(D, st), "dense_scan launch");
-    return;
-  }
-  if (B->ring) {
-    run_ring(B, grad, keep, energy_out, grad_out, st);
     return;
   }
   launch_prep(B, st);
@@ -1759,8 +1765,7 @@ rsv_status run_in_workspace(int n, int L, double field, const double *d_params, 
     // amplitudes of the state buffers must start at zero.
     if (B.plan.phys > n)
       check(cudaMemsetAsync(B.states.p, 0, 3 * B.state_len * sizeof(double2), st), "state clear");
-    check(launch_coef(d_params, B.coef.p, static_cast<int>(nl), st), "coef launch");
-    run_all(&B, d_gradient_out != nullptr, d_energy_out, d_gradient_out, st);
+    run_all(&B, d_params, d_gradient_out != nullptr, d_energy_out, d_gradient_out, st);
     // nothing enqueued above refers to host memory of this call
   });
 }
@@ -1878,12 +1883,50 @@ void assign_energy_fusion(rsv_backend *B) {
   assign_energy_deferral(B);
 }
 
+// Which circuits are contracted along the ring, at a cost of n 16^(L-1) L against
+// 2^n n L for the state.  Up to 4 layers the cluster-resident state is the
+// faster one below 12 qubits (L = 4, energy and gradient: n = 10 18 us against
+// 25, n = 12 37 against 27), and the tile passes never are (n = 12 142 us, n =
+// 28 21 400 against 38).  5 layers cross the cluster at n = 16 (191 us against
+// 180; n = 15 115 against 175).
+bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 16 && L == 5); }
+
+// How a single circuit is spread over a cluster (rsv_cluster.cu), the fastest of
+// the measured shapes at L = 8: up to 9 qubits 4 amplitudes a thread on one
+// CTA (n = 9 23.6 us, 8 a thread 24.8, 16 a thread 47), 10 and 11 qubits 8 a
+// thread (31 and 51 us; 4 a thread 35 and 55), 12 and 13 on 8 CTAs (64 and 86
+// us; on one or two 90 and 180), then 16 CTAs (14 qubits 120 us against 137 on
+// 8, 16 qubits 293 against 336 on the tile passes).
+ClusterShape cluster_shape_for(int n) {
+  if (n <= 9) return {0, 2};
+  if (n <= 11) return {0, 3};
+  if (n <= 13) return {3, 3};
+  return {4, 4};
+}
+
+// What runs a backend's calls.  A caller that chose a backward schedule, fewer
+// analytic layers or other kernels chose a tile-pass plan; the defaults choose
+// by the circuit.
+Path choose_path(rsv_backend *B, int mode) {
+  const bool defaults = mode == RSV_BACKWARD_AUTO && B->analytic_layers == kDefaultAnalyticLayers &&
+                        B->kernel_flags == (RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY) && B->force_c == 0;
+  if (!defaults || B->dense || B->gate_level) return Path::kPasses;
+  if (ring_rule(B->n, B->L)) return Path::kRing;
+  if (B->n > kClusterMaxQubits || B->L > kClusterMaxLayers) return Path::kPasses;
+  B->cluster_shape = cluster_shape_for(B->n);
+  int clusters = 0;
+  if (cluster_capacity(B->n, B->cluster_shape, B->L, &clusters) != cudaSuccess)
+    cudaGetLastError();  // such a cluster does not fit this device
+  if (clusters >= 1) return Path::kCluster;
+  return Path::kPasses;
+}
+
 void assign_backward_kernels(rsv_backend *B) {
   B->tma.assign(B->plan.bwd.size(), TmaPass{});
   B->tma_passes = 0;
   if (B->pipeline_err.p == nullptr) {
-    B->pipeline_err.alloc(1);
-    check(cudaMemset(B->pipeline_err.p, 0, sizeof(int)), "pipeline flag clear");
+    B->pipeline_err.alloc(2 + kMaxQubits);
+    check(cudaMemset(B->pipeline_err.p, 0, (2 + kMaxQubits) * sizeof(int)), "pipeline flag clear");
   }
   PassParams P;
   for (size_t i = 0; i < B->plan.bwd.size(); ++i) {
@@ -1913,7 +1956,19 @@ void setup_plan(rsv_backend *B, int mode) {
   B->states.release();
   Plan pl = make_plan(B->n, B->L, B->sms, want, B->analytic_layers, B->force_c);
   B->state_len = size_t{1} << pl.phys;
-  try {
+  B->path = choose_path(B, mode);
+  const size_t ring_values =
+      B->path == Path::kRing ? 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs : 0;
+  if (ring_values > static_cast<size_t>(pl.num_bufs) * B->state_len) {
+    try {
+      B->states.alloc(ring_values);
+    } catch (const Error &e) {
+      if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
+      cudaGetLastError();  // clear the allocation failure
+      B->path = Path::kPasses;
+    }
+  }
+  if (B->states.p == nullptr) try {
     B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
   } catch (const Error &e) {
     if (mode != RSV_BACKWARD_AUTO || !pl.checkpoint || e.status != RSV_ERR_OUT_OF_MEMORY) throw;
@@ -1921,7 +1976,10 @@ void setup_plan(rsv_backend *B, int mode) {
     pl = make_plan(B->n, B->L, B->sms, false, B->analytic_layers, B->force_c);
     B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
   }
-  check(cudaMemset(B->states.p, 0, B->states.count * sizeof(double2)), "state memset");
+  // (zero padding for n < 12; the ring's components need none)
+  check(cudaMemset(B->states.p, 0, std::min(B->states.count, static_cast<size_t>(pl.num_bufs) * B->state_len) *
+                                       sizeof(double2)),
+        "state memset");
   B->plan = pl;
   B->backward_mode = mode;
   B->num_bwd_passes = static_cast<int>(B->plan.bwd.size());
@@ -1970,7 +2028,6 @@ void setup_plan(rsv_backend *B, int mode) {
 struct TuneChoice {
   int mode = RSV_BACKWARD_AUTO, analytic = kDefaultAnalyticLayers;
   int kernels = RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY, force_c = 0;
-  bool ring = false;  // contraction along the ring instead of a tile-pass plan
   double ms = 0.0;
 };
 
@@ -1989,12 +2046,11 @@ void apply_choice(rsv_backend *B, const TuneChoice &c) {
   B->kernel_flags = c.kernels;
   B->force_c = c.force_c;
   setup_plan(B, c.mode);
-  if (c.ring) setup_ring(B);
-  else leave_ring(B);
 }
 
 std::string choice_str(const rsv_backend *B, const TuneChoice &c) {
-  if (c.ring) return "ring contraction";
+  if (B->path == Path::kRing) return "ring contraction";
+  if (B->path == Path::kCluster) return "cluster-resident state";
   std::ostringstream os;
   os << "mode=" << (B->plan.checkpoint ? "checkpoint" : "uncompute") << " analytic_layers=" << c.analytic
      << " tma=" << ((c.kernels & RSV_KERNELS_TMA) ? 1 : 0) << " tma_passes=" << B->tma_passes
@@ -2005,16 +2061,13 @@ std::string choice_str(const rsv_backend *B, const TuneChoice &c) {
 
 // Mean milliseconds of one energy_and_grad of the current plan (one untimed call first).
 double time_plan(rsv_backend *B, const double *d_params, int repeats, cudaStream_t st) {
-  const int nl = B->n * B->L;
-  check(launch_coef(d_params, B->coef.p, nl, st), "coef launch");
-  run_all(B, true, B->outputs.p, B->outputs.p + 1, st);
+  run_all(B, d_params, true, B->outputs.p, B->outputs.p + 1, st);
   cudaEvent_t a, b;
   check(cudaEventCreate(&a), "cudaEventCreate");
   check(cudaEventCreate(&b), "cudaEventCreate");
   check(cudaEventRecord(a, st), "cudaEventRecord");
   for (int r = 0; r < repeats; ++r) {
-    check(launch_coef(d_params, B->coef.p, nl, st), "coef launch");
-    run_all(B, true, B->outputs.p, B->outputs.p + 1, st);
+    run_all(B, d_params, true, B->outputs.p, B->outputs.p + 1, st);
   }
   check(cudaEventRecord(b, st), "cudaEventRecord");
   check(cudaEventSynchronize(b), "autotune synchronize");
@@ -2025,18 +2078,14 @@ double time_plan(rsv_backend *B, const double *d_params, int repeats, cudaStream
   return static_cast<double>(ms) / repeats;
 }
 
-// The candidates: the ring contraction where the rule takes it, then the
-// tile-pass plans: both backward schedules (checkpoint only where it fits),
+// The candidates: what the defaults choose where that is not a tile-pass plan,
+// then the tile-pass plans: both backward schedules (checkpoint only where it fits),
 // three or two analytic leading layers, the TMA kernels on (with or without
 // the fused energy) or off, and every
 // contiguous run length c of the high tiles that gives the fewest passes.
-std::vector<TuneChoice> tune_candidates(const rsv_backend *B) {
+std::vector<TuneChoice> tune_candidates(const rsv_backend *B, bool direct) {
   std::vector<TuneChoice> out;
-  if (ring_rule(B->n, B->L)) {
-    TuneChoice t;
-    t.ring = true;
-    out.push_back(t);
-  }
+  if (direct) out.push_back(TuneChoice{});
   std::vector<int> cs = {0};
   if (B->n > 12) {
     auto passes = [&](int c) { return static_cast<int>(high_tiles(B->n, 12, 2, c).size()); };
@@ -2157,7 +2206,6 @@ rsv_status rsv_create(int num_qubits, int num_layers, double field, const char *
       B->gate_grid = gate_grid(num_qubits, B->sms);
       B->gate_partials.alloc(static_cast<size_t>(B->gate_grid) * (1 + 2 * nl));
     }
-    refresh_ring(B.get());
     B->coef.alloc(nl);
     B->ptab.alloc(static_cast<size_t>(num_layers) * 1024);
     B->outputs.alloc(1 + B->num_params);
@@ -2197,11 +2245,16 @@ rsv_status rsv_energy_and_grad(rsv_backend *B, const double *params, size_t num_
     cudaStream_t st = pick_stream(B, stream);
     upload_host_coefs(B, params, st);
     const bool grad = compute_gradient != 0;
-    run_all(B, grad, B->outputs.p, B->outputs.p + 1, st);
-    const size_t count = grad ? 1 + B->num_params : 1;
-    check(cudaMemcpyAsync(B->out_host.p, B->outputs.p, count * sizeof(double),
-                          cudaMemcpyDeviceToHost, st),
-          "result download");
+    if (B->path != Path::kPasses) {
+      // the kernels write their few results straight into pinned host memory
+      run_all(B, nullptr, grad, B->out_host.p, B->out_host.p + 1, st);
+    } else {
+      run_all(B, nullptr, grad, B->outputs.p, B->outputs.p + 1, st);
+      const size_t count = grad ? 1 + B->num_params : 1;
+      check(cudaMemcpyAsync(B->out_host.p, B->outputs.p, count * sizeof(double),
+                            cudaMemcpyDeviceToHost, st),
+            "result download");
+    }
     check(cudaStreamSynchronize(st), "energy_and_grad");
     check_pipeline(B, B->out_host.p[0]);
     *energy_out = B->out_host.p[0];
@@ -2216,10 +2269,7 @@ rsv_status rsv_energy_and_grad_device(rsv_backend *B, const double *d_params, si
     validate_params(B, d_params, num_params);
     if (d_energy_out == nullptr) invalid("d_energy_out is null");
     cudaStream_t st = device_stream(stream);
-    timed(B, st, 0, 0.0, [&] {
-      check(launch_coef(d_params, B->coef.p, static_cast<int>(B->n * B->L), st), "coef launch");
-    });
-    run_all(B, d_gradient_out != nullptr, d_energy_out, d_gradient_out, st);
+    run_all(B, d_params, d_gradient_out != nullptr, d_energy_out, d_gradient_out, st);
   });
 }
 
@@ -2231,8 +2281,7 @@ rsv_status rsv_forward_device(rsv_backend *B, const double *d_params, size_t num
     validate_params(B, d_params, num_params);
     if (d_energy_out == nullptr) invalid("d_energy_out is null");
     cudaStream_t st = device_stream(stream);
-    check(launch_coef(d_params, B->coef.p, static_cast<int>(B->n * B->L), st), "coef launch");
-    run_all(B, false, d_energy_out, nullptr, st, true);
+    run_all(B, d_params, false, d_energy_out, nullptr, st, true);
     B->forward_only_state = true;
     if (generation_out) *generation_out = B->generation;
   });
@@ -2248,8 +2297,8 @@ rsv_status rsv_backward_device(rsv_backend *B, unsigned long long generation,
       throw Error(RSV_ERR_STALE_STATE,
                   "backward needs the state of the matching forward; the backend ran another call since");
     cudaStream_t st = device_stream(stream);
-    if (B->ring) {
-      run_ring_backward(B, d_gradient_out, st);
+    if (B->path != Path::kPasses) {
+      run_direct_backward(B, d_gradient_out, st);
     } else {
       run_backward(B, st, false);  // the forward call computed the whole energy
       // energy is rewritten with the same value into the outputs scratch slot
@@ -2285,19 +2334,27 @@ rsv_status rsv_profile_energy_and_grad(rsv_backend *B, const double *params, siz
       // one stage: these schedules are not split into the phases below
       cudaEventRecord(ev[1], st);
       --B->generation;  // run_all counts the call
-      run_all(B, grad, B->outputs.p, B->outputs.p + 1, st);
+      run_all(B, nullptr, grad, B->outputs.p, B->outputs.p + 1, st);
       cudaEventRecord(ev[2], st);
       cudaEventRecord(ev[3], st);
       cudaEventRecord(ev[4], st);
-    } else if (B->ring) {
+    } else if (B->path == Path::kRing) {
       // the sweeps (energy included) as the forward stage, the gradient as the backward
-      B->ring_field = B->field;
-      const RingParams R = ring_params(B, B->outputs.p, B->outputs.p + 1);
+      B->forward_field = B->field;
+      const RingParams R = ring_params(B, nullptr, B->outputs.p, B->outputs.p + 1);
       cudaEventRecord(ev[1], st);
       check(launch_ring_sweeps(R, true, grad, grad, st), "ring sweep launch");
       cudaEventRecord(ev[2], st);
       cudaEventRecord(ev[3], st);
       if (grad) check(launch_ring_gradient(R, st), "ring gradient launch");
+      cudaEventRecord(ev[4], st);
+    } else if (B->path == Path::kCluster) {
+      // the same work in two launches: forward and energy, then the backward
+      cudaEventRecord(ev[1], st);
+      run_direct(B, nullptr, false, true, B->outputs.p, nullptr, st);
+      cudaEventRecord(ev[2], st);
+      cudaEventRecord(ev[3], st);
+      if (grad) run_direct_backward(B, B->outputs.p + 1, st);
       cudaEventRecord(ev[4], st);
     } else {
       launch_prep(B, st);
@@ -2426,7 +2483,6 @@ rsv_status rsv_set_backward_mode(rsv_backend *B, int mode) {
     if (B == nullptr) invalid("backend is null");
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     setup_plan(B, mode);
-    refresh_ring(B);
   });
 }
 
@@ -2438,7 +2494,6 @@ rsv_status rsv_set_analytic_layers(rsv_backend *B, int max_layers) {
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     B->analytic_layers = max_layers;
     setup_plan(B, B->backward_mode);
-    refresh_ring(B);
   });
 }
 
@@ -2450,7 +2505,6 @@ rsv_status rsv_set_kernels(rsv_backend *B, int flags) {
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     B->kernel_flags = flags;
     setup_plan(B, B->backward_mode);
-    refresh_ring(B);
   });
 }
 
@@ -2484,7 +2538,7 @@ rsv_status rsv_autotune(rsv_backend *B, const double *d_params, size_t num_param
       }
     }
     std::ostringstream rep;
-    const TuneChoice before{B->backward_mode, B->analytic_layers, B->kernel_flags, B->force_c, B->ring, 0.0};
+    const TuneChoice before{B->backward_mode, B->analytic_layers, B->kernel_flags, B->force_c, 0.0};
     TuneChoice best;
     best.ms = 1e300;
     std::vector<std::string> seen;
@@ -2492,7 +2546,15 @@ rsv_status rsv_autotune(rsv_backend *B, const double *d_params, size_t num_param
     // deviation from the first candidate's outputs is reported
     std::vector<double> ref_out, cur_out(1 + B->num_params);
     double spread = 0.0;
-    for (TuneChoice c : tune_candidates(B)) {
+    bool direct = false;
+    try {
+      apply_choice(B, TuneChoice{});
+      direct = B->path != Path::kPasses;
+    } catch (const Error &e) {
+      if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
+      cudaGetLastError();
+    }
+    for (TuneChoice c : tune_candidates(B, direct)) {
       try {
         apply_choice(B, c);
       } catch (const Error &e) {
@@ -2502,7 +2564,7 @@ rsv_status rsv_autotune(rsv_backend *B, const double *d_params, size_t num_param
         continue;
       }
       // the same launches under another name are timed once
-      std::string sig = std::string(B->ring ? "ring " : "") + describe(B->plan) + " fused_energy=" + std::to_string(B->energy_fuse_pass) +
+      std::string sig = std::string(B->path != Path::kPasses ? "direct " : "") + describe(B->plan) + " fused_energy=" + std::to_string(B->energy_fuse_pass) +
                         std::to_string(B->energy_defer_pass);
       if (std::find(seen.begin(), seen.end(), sig) != seen.end()) continue;
       seen.push_back(sig);
@@ -2537,7 +2599,9 @@ rsv_status rsv_describe_backend(rsv_backend *B, char *buf, size_t buf_size, size
     os << "analytic_layers=" << B->analytic_layers << " kernels=" << B->kernel_flags
        << " high_tile_c=" << (B->force_c ? std::to_string(B->force_c) : std::string("planner"))
        << " tma_passes=" << B->tma_passes;
-    if (B->ring) os << " ring_contraction (the plan below is not used)";
+    if (B->path == Path::kRing) os << " ring_contraction (the plan below is not used)";
+    if (B->path == Path::kCluster)
+      os << " cluster_resident: " << (1 << B->cluster_shape.log_ctas) << " CTAs x " << (1 << B->cluster_shape.register_bits) << " amplitudes (the plan below is not used)";
     if (B->energy_fuse_pass >= 0)
       os << " fused_energy: backward pass " << B->energy_fuse_pass << " applies "
          << kTmaNumEnergyMasks << " field terms,"

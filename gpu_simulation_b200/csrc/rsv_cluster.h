@@ -1,0 +1,49 @@
+// Circuits whose state lives in the registers and shared memory of one
+// thread-block cluster (rsv_cluster.cu): host-callable launchers.
+#pragma once
+
+#include <cstddef>
+#include <cuda_runtime.h>
+
+namespace rsv {
+
+constexpr int kClusterMaxQubits = 16;
+constexpr int kClusterMaxLayers = 64;
+
+// One circuit of a launch; every circuit of a launch has n qubits.
+struct ClusterItem {
+  int L;
+  int index;              // energy_out[index]
+  long long param_off;    // params, grad_out: + param_off
+  double h;
+};
+
+struct ClusterArgs {
+  int n;
+  int log_ctas;                // CTAs of a cluster (= of a circuit): 2^log_ctas
+  int register_bits;           // amplitudes of a thread: 2^register_bits
+  int count;                   // circuits
+  const ClusterItem *items;    // [count], or null: the one circuit `item`
+  ClusterItem item;
+  int max_layers;              // largest L of the circuits
+  const double *params;        // angles, or null: `coef` (one circuit)
+  const double4 *coef;         // [L * n] (cos t/2, sin t/2, cos p/2, sin p/2)
+  double4 *coef_out;           // or null: the one circuit's are written here
+  double *energy_out;          // or null
+  double *grad_out;            // or null: no backward
+  // One circuit only: the forward call leaves psi and H psi here, and with
+  // `resume` a later call starts from them and runs the backward alone.
+  double2 *psi, *lam;
+  int resume;
+};
+
+// How a launch spreads a circuit: 2^log_ctas CTAs, 2^register_bits amplitudes a thread.
+struct ClusterShape {
+  int log_ctas, register_bits;
+};
+bool cluster_shape_built(int n, ClusterShape h);
+cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s);
+// Clusters of that shape that fit the device at once (0: none).
+cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *clusters);
+
+}  // namespace rsv

@@ -19,7 +19,8 @@
 //   I identity so far, X an open X on the last wire, H complete terms,
 //   W an open X_0 X_1, S the Z string.
 // The ring is closed by fixing the bits (a, abar) that enter wire 0: D^2
-// independent chains, each a D x D matrix (ket bits x bra bits) per component.
+// independent chains, each a D x D matrix (ket bits x bra bits) per component;
+// (abar, a) has the conjugate transposes of (a, abar), so D (D + 1) / 2 are carried.
 // Exact, and the cost is n 16^(L-1) L instead of 2^n n L; every entry is a
 // transition amplitude between projected states, at most 1 in magnitude, so
 // nothing grows along the chain.
@@ -33,15 +34,11 @@
 //     shuffle (element j of a lane is k = 2 (lane % 4) + j of the operand), and
 //     the second product's accumulator is again ket x bra.  A sixth warp
 //     builds the next site's T.  One barrier per site.
-//   ring_grad_kernel: one cluster per site.  From the left components before
+//   ring_grad_kernel: up to eight CTAs a site.  From the left components before
 //     and the right components after the site: dE/dT[s; s'] summed over chains
 //     and components on the tensor cores, then the site's 2 L derivatives.
 // Both are bound by latency (n dependent sites of two small products), not by
 // memory or arithmetic throughput.
-// energy_and_grad at L = 4: n = 16 33 us (tile passes 141), n = 24 40 us (1598),
-// n = 28 42 us (21 400).  L = 5 (16 x 16 matrices): n = 22 427 us (807), n = 24
-// 445 us (2631); n = 20 410 us against 322.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -53,84 +50,82 @@
 namespace rsv {
 namespace {
 
-namespace cg = cooperative_groups;
-
 constexpr int kComps = 5;  // I, X, H, W, S
 constexpr int kI = 0, kX = 1, kH = 2, kW = 3, kS = 4;
 constexpr int kSweepThreads = 32 * (kComps + 1);
-constexpr int kGradWarps = 8;
-constexpr int kMaxDerivs = 2 * kRingMaxLayers;
+constexpr int kGradWarps = 2 * kComps;
+constexpr int kMaxDerivs = kRingDerivs;
 
 struct SiteM {  // cos, sin of the full angles of a wire's last layer
   double ct, st, cp, sp;
 };
 
-// A D x D complex matrix in a warp's registers: tile (i, j), element e of lane
-// l is row 8 i + l / 4, column 8 j + 2 (l % 4) + e.
-template <int DB>
+// An 8 R x 8 C complex matrix in a warp's registers: tile (i, j), element e of
+// lane l is row 8 i + l / 4, column 8 j + 2 (l % 4) + e.
+template <int R, int C>
 struct Mat {
-  double re[DB][DB][2], im[DB][DB][2];
+  double re[R][C][2], im[R][C][2];
 };
 
+__device__ __forceinline__ int frag_row(int i, int lane) { return 8 * i + lane / 4; }
+__device__ __forceinline__ int frag_col(int j, int lane, int e) { return 8 * j + 2 * (lane % 4) + e; }
+// D x D matrices in memory keep that order, [tile][element][lane] (D = 8 DB):
+// where element (row, col) is.
 template <int DB>
-__device__ __forceinline__ int frag_row(int i, int lane) {
-  return 8 * i + lane / 4;
-}
-template <int DB>
-__device__ __forceinline__ int frag_col(int j, int lane, int e) {
-  return 8 * j + 2 * (lane % 4) + e;
+__device__ __forceinline__ int frag_at(int row, int col) {
+  return (row / 8 * DB + col / 8) * 64 + 32 * (col & 1) + (row % 8) * 4 + (col % 8) / 2;
 }
 
+template <int R, int C, typename F>
+__device__ __forceinline__ void elements(F &&f) {
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) f(i, j, e);
+}
+
+template <int R, int C>
+__device__ __forceinline__ Mat<R, C> zero_mat() {
+  Mat<R, C> m;
+  elements<R, C>([&](int i, int j, int e) { m.re[i][j][e] = m.im[i][j][e] = 0.0; });
+  return m;
+}
 template <int DB>
-__device__ __forceinline__ Mat<DB> zero_mat() {
-  Mat<DB> m;
-#pragma unroll
-  for (int i = 0; i < DB; ++i)
-#pragma unroll
-    for (int j = 0; j < DB; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) m.re[i][j][e] = m.im[i][j][e] = 0.0;
+__device__ __forceinline__ void store_mat(double2 *p, const Mat<DB, DB> &m, int lane) {
+  elements<DB, DB>([&](int i, int j, int e) {
+    p[(i * DB + j) * 64 + 32 * e + lane] = make_double2(m.re[i][j][e], m.im[i][j][e]);
+  });
+}
+template <int DB>
+__device__ __forceinline__ Mat<DB, DB> load_mat(const double2 *p, int lane) {
+  Mat<DB, DB> m;
+  elements<DB, DB>([&](int i, int j, int e) {
+    const double2 v = p[(i * DB + j) * 64 + 32 * e + lane];
+    m.re[i][j][e] = v.x;
+    m.im[i][j][e] = v.y;
+  });
   return m;
 }
 
-// Matrices in memory keep that order: [tile][lane][element].
-template <int DB>
-__device__ __forceinline__ void store_mat(double2 *p, const Mat<DB> &m, int lane) {
+// Z[m][n] += sum_k A[m][k] B[n][k], A conjugated when CONJ; of Z's tiles only
+// those with m == n when OUTD, and only B's tiles with n == k when BD, A's
+// with m == k when AD (the others are zero).  `n0`: the tile row of B that its
+// first one is.
+template <bool CONJ, bool OUTD, bool BD, bool AD, int R, int C, int K>
+__device__ __forceinline__ void mma_rows(Mat<R, C> &Z, const Mat<R, K> &A, const Mat<C, K> &B, int n0 = 0) {
 #pragma unroll
-  for (int i = 0; i < DB; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int j = 0; j < DB; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        p[(i * DB + j) * 64 + 2 * lane + e] = make_double2(m.re[i][j][e], m.im[i][j][e]);
-}
-template <int DB>
-__device__ __forceinline__ Mat<DB> load_mat(const double2 *p, int lane) {
-  Mat<DB> m;
-#pragma unroll
-  for (int i = 0; i < DB; ++i)
-#pragma unroll
-    for (int j = 0; j < DB; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double2 v = p[(i * DB + j) * 64 + 2 * lane + e];
-        m.re[i][j][e] = v.x;
-        m.im[i][j][e] = v.y;
-      }
-  return m;
-}
-
-// Z[m][n] += sum_k A[m][k] B[n][k] (no conjugation of B; A conjugated when CONJ).
-template <int DB, bool CONJ>
-__device__ __forceinline__ void mma_rows(Mat<DB> &Z, const Mat<DB> &A, const Mat<DB> &B) {
-#pragma unroll
-  for (int i = 0; i < DB; ++i)
-#pragma unroll
-    for (int j = 0; j < DB; ++j) {
+    for (int j = 0; j < C; ++j) {
+      if (OUTD && i != j) continue;
       double r0 = Z.re[i][j][0], r1 = Z.re[i][j][1], q0 = 0.0, q1 = 0.0;
       double s0 = Z.im[i][j][0], s1 = Z.im[i][j][1], t0 = 0.0, t1 = 0.0;
 #pragma unroll
-      for (int k = 0; k < DB; ++k)
+      for (int k = 0; k < K; ++k) {
+        if (BD && j + n0 != k) continue;
+        if (AD && i != k) continue;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           mma_f64(r0, r1, A.re[i][k][e], B.re[j][k][e]);
@@ -138,6 +133,7 @@ __device__ __forceinline__ void mma_rows(Mat<DB> &Z, const Mat<DB> &A, const Mat
           mma_f64(s0, s1, A.re[i][k][e], B.im[j][k][e]);
           mma_f64(t0, t1, A.im[i][k][e], B.re[j][k][e]);
         }
+      }
       Z.re[i][j][0] = CONJ ? r0 + q0 : r0 - q0;
       Z.re[i][j][1] = CONJ ? r1 + q1 : r1 - q1;
       Z.im[i][j][0] = CONJ ? s0 - t0 : s0 + t0;
@@ -145,16 +141,26 @@ __device__ __forceinline__ void mma_rows(Mat<DB> &Z, const Mat<DB> &A, const Mat
     }
 }
 
-// T . V . T^+ for T given as rows of the result's side: first the bra columns
-// (conj T), then the ket rows; `T` is in shared memory in matrix order.
-template <int DB>
-__device__ __forceinline__ Mat<DB> sandwich(const double2 *T, const Mat<DB> &V, int lane) {
-  const Mat<DB> t = load_mat<DB>(T, lane);
-  Mat<DB> z = zero_mat<DB>();
-  mma_rows<DB, true>(z, t, V);   // z[bra][ket]
-  Mat<DB> y = zero_mat<DB>();
-  mma_rows<DB, false>(y, t, z);  // y[ket][bra]
+// T . V . T^+: first the bra columns (conj T), then the ket rows; `T` is in
+// shared memory in matrix order.  IND: V's off-diagonal tiles are zero; OUTD:
+// only the result's diagonal tiles are wanted (the others come back zero).
+template <int DB, bool IND, bool OUTD>
+__device__ __forceinline__ Mat<DB, DB> sandwich(const double2 *T, const Mat<DB, DB> &V, int lane) {
+  const Mat<DB, DB> t = load_mat<DB>(T, lane);
+  Mat<DB, DB> z = zero_mat<DB, DB>();
+  mma_rows<true, false, IND, false>(z, t, V);   // z[bra][ket]
+  Mat<DB, DB> y = zero_mat<DB, DB>();
+  mma_rows<false, OUTD, false, false>(y, t, z);  // y[ket][bra]
   return y;
+}
+template <int DB>
+__device__ __forceinline__ Mat<DB, DB> sandwich(const double2 *T, const Mat<DB, DB> &V, bool ind, bool outd, int lane) {
+  if constexpr (DB > 1) {
+    if (ind && outd) return sandwich<DB, true, true>(T, V, lane);
+    if (ind) return sandwich<DB, true, false>(T, V, lane);
+    if (outd) return sandwich<DB, false, true>(T, V, lane);
+  }
+  return sandwich<DB, false, false>(T, V, lane);
 }
 
 __device__ __forceinline__ SiteM site_m(double4 c) {
@@ -212,9 +218,17 @@ __device__ __forceinline__ double2 t0_entry(const double2 *U, int stride, int nb
 // Element e of a matrix in memory order is row r, column c of it.
 template <int DB>
 __device__ __forceinline__ void order_rc(int e, int &r, int &c) {
-  const int tile = e / 64, lane = (e % 64) / 2;
-  r = frag_row<DB>(tile / DB, lane);
-  c = frag_col<DB>(tile % DB, lane, e & 1);
+  const int tile = e / 64, lane = e % 32;
+  r = frag_row(tile / DB, lane);
+  c = frag_col(tile % DB, lane, (e / 32) & 1);
+}
+
+// Chain k is the k-th pair a <= ab (by ab, then a); the pair (ab, a) has the
+// conjugate transposes of its matrices and is not carried.
+__device__ __forceinline__ void chain_pair(int k, int &a, int &ab) {
+  ab = 0;
+  while ((ab + 1) * (ab + 2) / 2 <= k) ++ab;
+  a = k - ab * (ab + 1) / 2;
 }
 
 // The bit of a bond index that is the wire's value before the last layer.
@@ -226,17 +240,14 @@ constexpr size_t sweep_smem_bytes(int n, int L) {
          sizeof(SiteM) * static_cast<size_t>(n);
 }
 
-// Applies f(i, j, e, bra bit, ket bit) to every element of a lane; the bits are
-// those before the last layer, flipped by fb / fk (wire 0: the arriving bits).
-template <int DB, typename F>
-__device__ __forceinline__ void each(int lane, int nb, int fk, int fb, F &&f) {
-#pragma unroll
-  for (int i = 0; i < DB; ++i)
-#pragma unroll
-    for (int j = 0; j < DB; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        f(i, j, e, last_bit(frag_col<DB>(j, lane, e), nb) ^ fb, last_bit(frag_row<DB>(i, lane), nb) ^ fk);
+// Applies f(i, j, e, bra bit, ket bit) to every element of a lane (tile rows
+// from i0); the bits are those before the last layer, flipped by fb / fk (wire
+// 0: the arriving bits).
+template <int R, int C, typename F>
+__device__ __forceinline__ void each(int lane, int nb, int fk, int fb, F &&f, int i0 = 0) {
+  elements<R, C>([&](int i, int j, int e) {
+    f(i, j, e, last_bit(frag_col(j, lane, e), nb) ^ fb, last_bit(frag_row(i0 + i, lane), nb) ^ fk);
+  });
 }
 
 // Left components after a site from those before its last layer (t*), for
@@ -247,16 +258,31 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
   constexpr int D = 8 * DB, DD = D * D;
   extern __shared__ double2 smem[];
   const int n = P.n, L = P.L, nb = L - 1;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int chains = gridDim.x, chain = blockIdx.x;
   const bool rightward = first_dir + static_cast<int>(blockIdx.y) == 0;
-  const int a = chain >> nb, ab = chain & ((1 << nb) - 1);
+  int a, ab;
+  chain_pair(chain, a, ab);
   double2 *U = smem;                       // [nb][n][4]
   double2 *T = U + nb * n * 4;             // [2][DD]
   double2 *ex = T + 2 * DD;                // [2][3][DD]
   SiteM *M = reinterpret_cast<SiteM *>(ex + 6 * DD);  // [n]
-  const int tid = threadIdx.x, lane = tid & 31, comp = tid >> 5;
-  for (int k = tid; k < nb * n; k += kSweepThreads) site_u(P.coef[k], U + 4 * k);
-  for (int k = tid; k < n; k += kSweepThreads) M[k] = site_m(P.coef[nb * n + k]);
+  const int tid = threadIdx.x, lane = tid & 31;
+  // W and I, the components with the fewest products, share a scheduler
+  constexpr int kCompOf[kComps + 1] = {kW, kH, kX, kS, kI, kComps};
+  const int comp = kCompOf[tid >> 5];
+  for (int k = tid; k < L * n; k += kSweepThreads) {
+    double4 v;
+    if (P.params) {
+      sincos(P.params[2 * k] * 0.5, &v.y, &v.x);
+      sincos(P.params[2 * k + 1] * 0.5, &v.w, &v.z);
+      if (blockIdx.x == 0 && blockIdx.y == 0) P.coef[k] = v;  // for the gradient kernel
+    } else {
+      v = P.coef[k];
+    }
+    if (k < nb * n) site_u(v, U + 4 * k);
+    else M[k - nb * n] = site_m(v);
+  }
   __syncthreads();
   const int ustride = 4 * n;
   auto build = [&](int w, double2 *out, int first, int step) {
@@ -270,12 +296,12 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
   const double h = P.field;
 
   if (rightward) {
-    Mat<DB> v;
+    Mat<DB, DB> v;
     if (comp < kComps) {
       const SiteM m = M[0];
-      each<DB>(lane, nb, last_bit(a, nb), last_bit(ab, nb), [&](int i, int j, int e, int bra, int ket) {
-        const double2 uk = t0_entry(U, ustride, nb, frag_row<DB>(i, lane), a);
-        const double2 ub = t0_entry(U, ustride, nb, frag_col<DB>(j, lane, e), ab);
+      each<DB, DB>(lane, nb, last_bit(a, nb), last_bit(ab, nb), [&](int i, int j, int e, int bra, int ket) {
+        const double2 uk = t0_entry(U, ustride, nb, frag_row(i, lane), a);
+        const double2 ub = t0_entry(U, ustride, nb, frag_col(j, lane, e), ab);
         double2 x = cmul_conj(uk, ub);
         if (comp == kI) {
           if (bra != ket) x = make_double2(0.0, 0.0);
@@ -295,8 +321,13 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
     for (int w = 1; w < n; ++w) {
       const int p = (w - 1) & 1;
       double2 *xI = ex + p * 3 * DD, *xX = xI + DD;
+      const SiteM m = M[w];
       if (comp < kComps) {
-        v = sandwich<DB>(T + p * DD, v, lane);
+        // behind an identity the bra and ket bits agree (at L = 5 the
+        // off-diagonal tiles are zero), and of H and W only what the next
+        // identity keeps is used
+        v = sandwich<DB>(T + p * DD, v, (comp == kI && w > 1) || (comp == kW && w > 2),
+                         comp == kH || (comp == kW && w < n - 1), lane);
         if (keep) store_mat<DB>(P.left + ((static_cast<size_t>(w) * chains + chain) * kComps + comp) * DD, v, lane);
         if (comp == kI) store_mat<DB>(xI, v, lane);
         if (comp == kX) store_mat<DB>(xX, v, lane);
@@ -305,21 +336,20 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
       }
       __syncthreads();
       if (w == n - 1) break;
-      const SiteM m = M[w];
       if (comp == kI || (comp == kW && w > 1) || (comp == kS && w == 1)) {
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+        each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
           if (bra != ket) v.re[i][j][e] = v.im[i][j][e] = 0.0;
         });
       } else if (comp == kX || comp == kW) {
         const double2 *src = comp == kX ? xI : xX;
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-          const double2 x = cmul(m_x(m, bra, ket), src[(i * DB + j) * 64 + 2 * lane + e]);
+        each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+          const double2 x = cmul(m_x(m, bra, ket), src[(i * DB + j) * 64 + 32 * e + lane]);
           v.re[i][j][e] = x.x;
           v.im[i][j][e] = x.y;
         });
       } else if (comp == kH) {
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-          const int at = (i * DB + j) * 64 + 2 * lane + e;
+        each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+          const int at = (i * DB + j) * 64 + 32 * e + lane;
           const double2 x = cmul(m_x(m, bra, ket), xX[at]);
           const double z = w == 1 ? 0.0 : m_z(m, bra, ket);
           const double2 t = xI[at];
@@ -328,7 +358,7 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
           v.im[i][j][e] = keep_im - z * t.y - h * x.y;
         });
       } else if (comp == kS) {
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+        each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
           const double z = m_z(m, bra, ket);
           v.re[i][j][e] *= z;
           v.im[i][j][e] *= z;
@@ -339,8 +369,8 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
     __shared__ double share[kComps];
     if (comp < kComps) {
       const SiteM m = M[n - 1];
-      each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-        if (frag_row<DB>(i, lane) != a || frag_col<DB>(j, lane, e) != ab) return;
+      each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+        if (frag_row(i, lane) != a || frag_col(j, lane, e) != ab) return;
         const double re = v.re[i][j][e], im = v.im[i][j][e];
         double x;
         if (comp == kH) {
@@ -357,7 +387,8 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
     __syncthreads();
     __shared__ bool last;
     if (tid == 0) {
-      P.energy_parts[chain] = ((share[kI] + share[kX]) + (share[kH] + share[kW])) + share[kS];
+      const double s = ((share[kI] + share[kX]) + (share[kH] + share[kW])) + share[kS];
+      P.energy_parts[chain] = a == ab ? s : 2.0 * s;
       __threadfence();
       last = atomicInc(P.counter, static_cast<unsigned>(chains - 1)) == static_cast<unsigned>(chains - 1);
     }
@@ -376,10 +407,10 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
   }
 
   // Right sweep: components after site n - 1 are the closed end.
-  Mat<DB> v = zero_mat<DB>();
+  Mat<DB, DB> v = zero_mat<DB, DB>();
   if (comp == kH || comp == kS)
-    each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int, int) {
-      if (frag_row<DB>(i, lane) == a && frag_col<DB>(j, lane, e) == ab) v.re[i][j][e] = 1.0;
+    each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int, int) {
+      if (frag_row(i, lane) == a && frag_col(j, lane, e) == ab) v.re[i][j][e] = 1.0;
     });
   for (int w = n - 1; w >= 1; --w) {
     const int p = (n - 1 - w) & 1;
@@ -389,14 +420,14 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
     if (comp == kW && w == 1) store_mat<DB>(xW, v, lane);
     if (comp < kComps && w < n - 1)
       store_mat<DB>(P.right + ((static_cast<size_t>(w) * chains + chain) * kComps + comp) * DD, v, lane);
-    __syncthreads();
     const SiteM m = M[w];
+    __syncthreads();
     if (comp == kComps) {
       if (w > 1) build(w - 1, T + (p ^ 1) * DD, lane, 32);
       continue;
     }
-    each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-      const int at = (i * DB + j) * 64 + 2 * lane + e;
+    each<DB, DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
+      const int at = (i * DB + j) * 64 + 32 * e + lane;
       double re = v.re[i][j][e], im = v.im[i][j][e];
       const double z = m_z(m, bra, ket);
       if (comp == kI) {
@@ -425,28 +456,68 @@ __global__ void __launch_bounds__(kSweepThreads) ring_sweep_kernel(const RingPar
       v.re[i][j][e] = re;
       v.im[i][j][e] = im;
     });
-    v = sandwich<DB>(T + p * DD, v, lane);
+    v = sandwich<DB>(T + p * DD, v, comp == kH || (comp == kW && w < n - 1),
+                     (comp == kI && w > 1) || (comp == kW && w > 2), lane);
   }
   if (comp < kComps)
     store_mat<DB>(P.right + (static_cast<size_t>(chain) * kComps + comp) * DD, v, lane);
 }
 
-// One cluster per site; its warps share the chains.
+// Rows [8 i0, ...) of a D x D matrix in shared memory (matrix order), or of its
+// conjugate transpose; conjugated once more when `conj`.
+template <int DB, int R>
+__device__ __forceinline__ Mat<R, DB> load_rows(const double2 *p, bool mirror, int i0, bool conj, int lane) {
+  Mat<R, DB> m;
+  const int base = mirror ? 32 * ((lane / 4) & 1) + 8 * (lane % 4) + lane / 8 : lane;
+  const int di = mirror ? 64 : 64 * DB, dj = mirror ? 64 * DB : 64, de = mirror ? 4 : 32;
+  const double sign = mirror != conj ? -1.0 : 1.0;
+  elements<R, DB>([&](int i, int j, int e) {
+    const double2 v = p[base + (i0 + i) * di + j * dj + e * de];
+    m.re[i][j][e] = v.x;
+    m.im[i][j][e] = sign * v.y;
+  });
+  return m;
+}
+
+// Chains of one step of ring_grad_kernel: 256 elements of each matrix kind.
 template <int DB>
-__global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingParams P) {
-  constexpr int D = 8 * DB, DD = D * D;
+__host__ __device__ constexpr int chains_a_step() {
+  return DB == 1 ? 4 : 1;
+}
+
+__device__ __forceinline__ void copy16(double2 *to, const double2 *from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(to))),
+               "l"(from)
+               : "memory");
+}
+
+// A site's CTAs share the chains, NC at a time.  The chains'
+// left components before and at the site and their right components are staged
+// in shared memory (cp.async, one step ahead); all threads turn them into the
+// products' operands V_c (left, before the site) and R_c (right, behind the
+// site's last layer) and take that layer's sums; then the warps form
+//   y[s'][bra] = sum V[s'][.] conj(T[bra][.]),  dE/dT[s][s'] += sum R[s][bra] y[s'][bra]
+// on the tensor cores: a warp has one component, and at L <= 4 the chain's pair
+// (a, ab) or its mirror (ab, a), at L = 5 both and one of the two tile rows of s'.
+// (Operands formed by every warp for itself: 480 us at n = 20, L = 5.)
+template <int DB>
+__global__ void __launch_bounds__(32 * kGradWarps, 1) ring_grad_kernel(const RingParams P) {
+  constexpr int D = 8 * DB, DD = D * D, kSlices = kGradWarps / DB;
   extern __shared__ double2 smem[];
   __shared__ double2 Uw[4 * (kRingMaxLayers - 1)], U0[4 * (kRingMaxLayers - 1)];
   __shared__ double red[kGradWarps][kMaxDerivs];
-  __shared__ double total[kMaxDerivs];
-  double2 *T = smem;              // [DD] T_w, or T_0 for sites 0 and 1 behind it
-  double2 *T0 = T + DD;           // [DD]
-  double2 *G = T0 + DD;           // [kGradWarps][DD]
-  cg::cluster_group cluster = cg::this_cluster();
-  const int G_ctas = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
-  const int w = static_cast<int>(blockIdx.x) / G_ctas;
-  const int n = P.n, L = P.L, nb = L - 1, chains = 1 << (2 * nb), bond = 1 << nb;
+  double2 *T = smem;              // [DD] T_w
+  double2 *T0 = T + DD;           // [DD] T_0
+  double2 *G = T0 + DD;           // [kSlices][DD]
+  constexpr int NC = chains_a_step<DB>(), kSet = kComps * DD;
+  double2 *stages = G + kSlices * DD;   // [2][NC][3][kComps][DD]
+  double2 *ops = stages + 6 * NC * kSet;  // [NC][2][kComps][DD]
+  const int G_ctas = static_cast<int>(gridDim.x), rank = static_cast<int>(blockIdx.x), w = static_cast<int>(blockIdx.y);
+  const int n = P.n, L = P.L, nb = L - 1, bond = 1 << nb, chains = bond * (bond + 1) / 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < kSlices * DD; e += 32 * kGradWarps) G[e] = make_double2(0.0, 0.0);
+  // launched while the sweeps end: their results from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid < nb) {
     site_u(P.coef[tid * n + w], Uw + 4 * tid);
     site_u(P.coef[tid * n], U0 + 4 * tid);
@@ -458,41 +529,38 @@ __global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingPa
     T[e] = t_entry(Uw, 4, nb, r, c);
     T0[e] = t0_entry(U0, 4, nb, r, c);
   }
-  for (int e = tid; e < kGradWarps * DD; e += 32 * kGradWarps) G[e] = make_double2(0.0, 0.0);
   __syncthreads();
   const double h = P.field;
-  const SiteM m = site_m(P.coef[nb * n + w]);
+  const SiteM m = site_m(P.coef[nb * n + w]), m1 = site_m(P.coef[nb * n + (w > 0 ? w - 1 : 0)]);
   // d/dtheta and d/dphi of M_X and M_Z of this site
-  const SiteM mt{-m.st, m.ct, m.cp, 0.0};  // theta: M_X keeps its cos(phi) part
-  const SiteM mp{m.ct, m.st, -m.sp, m.cp}; // phi
+  const SiteM mt{-m.st, m.ct, m.cp, 0.0};   // theta: M_X keeps its cos(phi) part
+  const SiteM mp{m.ct, m.st, -m.sp, m.cp};  // phi
   double g_theta = 0.0, g_phi = 0.0;
-  auto right_of = [&](int c, int chain) {
-    return load_mat<DB>(P.right + ((static_cast<size_t>(w) * chains + chain) * kComps + c) * DD, lane);
-  };
-  auto last_layer = [&](int bra, int ket, double2 qx, double2 qz) {
-    const double2 xt = m_x(mt, bra, ket), xp = m_x(mp, bra, ket);
-    g_theta += xt.x * qx.x - xt.y * qx.y + m_z(mt, bra, ket) * qz.x;
-    g_phi += xp.x * qx.x - xp.y * qx.y;
-  };
+  const int worker = rank * kGradWarps + warp, workers = G_ctas * kGradWarps;
   if (w == 0) {
-    // T_0's column a from the chains (a, .): sum over the bra bits and over ab
-    for (int a = rank * kGradWarps + warp; a < bond; a += G_ctas * kGradWarps) {
+    // T_0's column a from the pairs (a, .): sum over the bra bits and over ab
+    const int share = workers / bond;  // warps a column
+    if (worker < share * bond) {
+      const int a = worker % bond;
       double gr[DB], gi[DB];
 #pragma unroll
       for (int i = 0; i < DB; ++i) gr[i] = gi[i] = 0.0;
-      for (int ab = 0; ab < bond; ++ab) {
-        const int chain = (a << nb) | ab;
-        const Mat<DB> rI = right_of(kI, chain), rX = right_of(kX, chain), rH = right_of(kH, chain),
-                      rS = right_of(kS, chain);
-        each<DB>(lane, nb, last_bit(a, nb), last_bit(ab, nb), [&](int i, int j, int e, int bra, int ket) {
-          const double2 uk = t0_entry(U0, 4, nb, frag_row<DB>(i, lane), a);
-          const double2 ub = t0_entry(U0, 4, nb, frag_col<DB>(j, lane, e), ab);
+      for (int ab = worker / bond; ab < bond; ab += share) {
+        const int lo = a < ab ? a : ab, hi = a < ab ? ab : a;
+        const double2 *right = P.right + static_cast<size_t>(hi * (hi + 1) / 2 + lo) * kSet;
+        const Mat<DB, DB> rI = load_rows<DB, DB>(right + kI * DD, a > ab, 0, false, lane);
+        const Mat<DB, DB> rX = load_rows<DB, DB>(right + kX * DD, a > ab, 0, false, lane);
+        const Mat<DB, DB> rH = load_rows<DB, DB>(right + kH * DD, a > ab, 0, false, lane);
+        const Mat<DB, DB> rS = load_rows<DB, DB>(right + kS * DD, a > ab, 0, false, lane);
+        each<DB, DB>(lane, nb, last_bit(a, nb), last_bit(ab, nb), [&](int i, int j, int e, int bra, int ket) {
+          const double2 uk = T0[frag_at<DB>(frag_row(i, lane), a)];
+          const double2 ub = T0[frag_at<DB>(frag_col(j, lane, e), ab)];
           const double2 x = make_double2(rX.re[i][j][e], rX.im[i][j][e]);
-          const double2 s = make_double2(-(rH.re[i][j][e] + rS.re[i][j][e]), -(rH.im[i][j][e] + rS.im[i][j][e]));
+          const double2 q = make_double2(-(rH.re[i][j][e] + rS.re[i][j][e]), -(rH.im[i][j][e] + rS.im[i][j][e]));
           const double z = m_z(m, bra, ket);
           double2 r = cmul(m_x(m, bra, ket), x);
-          r.x += z * s.x;
-          r.y += z * s.y;
+          r.x += z * q.x;
+          r.y += z * q.y;
           if (bra == ket) {
             r.x += rI.re[i][j][e];
             r.y += rI.im[i][j][e];
@@ -501,7 +569,10 @@ __global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingPa
           gr[i] += r.x;
           gi[i] += r.y;
           const double2 v = cmul_conj(uk, ub);
-          last_layer(bra, ket, cmul(v, x), cmul(v, s));
+          const double2 qx = cmul(v, x), qz = cmul(v, q);
+          const double2 xt = m_x(mt, bra, ket), xp = m_x(mp, bra, ket);
+          g_theta += xt.x * qx.x - xt.y * qx.y + m_z(mt, bra, ket) * qz.x;
+          g_phi += xp.x * qx.x - xp.y * qx.y;
         });
       }
 #pragma unroll
@@ -511,137 +582,117 @@ __global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingPa
           gr[i] += __shfl_xor_sync(0xffffffffu, gr[i], o);
           gi[i] += __shfl_xor_sync(0xffffffffu, gi[i], o);
         }
-        // element (row, a) in matrix order, in this warp's slice
-        if (lane % 4 == 0)
-          G[warp * DD + (i * DB + a / 8) * 64 + 2 * ((lane / 4) * 4 + (a % 8) / 2) + (a & 1)] =
-              make_double2(gr[i], gi[i]);
+        // element (row, a); the warps of a slice have different columns
+        if (lane % 4 == 0) G[(warp / DB) * DD + frag_at<DB>(frag_row(i, lane), a)] = make_double2(gr[i], gi[i]);
       }
     }
   } else {
-    Mat<DB> g = zero_mat<DB>();
-    const Mat<DB> t = load_mat<DB>(T, lane);
-    const SiteM m1 = site_m(P.coef[nb * n + w - 1]);
-    for (int chain = rank * kGradWarps + warp; chain < chains; chain += G_ctas * kGradWarps) {
-      const int a = chain >> nb, ab = chain & (bond - 1);
-      const double2 *before = P.left + (static_cast<size_t>(w - 1) * chains + chain) * kComps * DD;
-      const double2 *here = P.left + (static_cast<size_t>(w) * chains + chain) * kComps * DD;
-      Mat<DB> rH, rX = zero_mat<DB>();
-      if (w == n - 1) {
-        rH = zero_mat<DB>();
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int, int) {
-          if (frag_row<DB>(i, lane) == a && frag_col<DB>(j, lane, e) == ab) rH.re[i][j][e] = 1.0;
-        });
-      } else {
-        rH = right_of(kH, chain);
-        rX = right_of(kX, chain);
+    const int c = warp / 2, js = DB == 1 ? 0 : warp % 2;
+    const bool end = w == n - 1, first = w == 1, second = w == 2;
+    auto fetch = [&](int chain0, double2 *to) {
+      for (int k = 0; k < NC && chain0 + k < chains; ++k, to += 3 * kSet) {
+        const size_t chain = static_cast<size_t>(chain0 + k);
+        const double2 *before = P.left + (static_cast<size_t>(w - 1) * chains + chain) * kSet;
+        const double2 *here = P.left + (static_cast<size_t>(w) * chains + chain) * kSet;
+        const double2 *right = P.right + (static_cast<size_t>(w) * chains + chain) * kSet;
+        for (int e = tid; e < kSet; e += 32 * kGradWarps) {
+          if (!first) copy16(to + e, before + e);  // (site 0's are formed from T_0)
+          copy16(to + kSet + e, here + e);
+          if (!end) copy16(to + 2 * kSet + e, right + e);  // (the closed end's are 0 or 1)
+        }
       }
-#pragma unroll
-      for (int c = 0; c < kComps; ++c) {
-        if (c == kW && w == 1) continue;  // no open X_0 X_1 before wire 1
-        // left component before the site, from the previous site's
-        Mat<DB> v;
-        if (w == 1) {
-          each<DB>(lane, nb, last_bit(a, nb), last_bit(ab, nb), [&](int i, int j, int e, int bra, int ket) {
-            const int col = frag_col<DB>(j, lane, e);
-            // rows a / ab of T_0 (column index in matrix order)
-            const double2 uk = T0[(i * DB + a / 8) * 64 + 2 * ((lane / 4) * 4 + (a % 8) / 2) + (a & 1)];
-            const double2 ub = T0[(col / 8 * DB + ab / 8) * 64 + 2 * ((col % 8) * 4 + (ab % 8) / 2) + (ab & 1)];
-            double2 x = cmul_conj(uk, ub);
-            if (c == kI) {
-              if (bra != ket) x = make_double2(0.0, 0.0);
-            } else if (c == kX) {
-              x = cmul(m_x(m1, bra, ket), x);
-            } else {
-              const double z = -m_z(m1, bra, ket);
-              x = make_double2(z * x.x, z * x.y);
-            }
-            v.re[i][j][e] = x.x;
-            v.im[i][j][e] = x.y;
-          });
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int step = G_ctas * NC;
+    Mat<DB, 1> g = zero_mat<DB, 1>();
+    fetch(rank * NC, stages);
+    for (int chain0 = rank * NC, k = 0; chain0 < chains; chain0 += step, ++k) {
+      const double2 *stage = stages + (k & 1) * 3 * NC * kSet;
+      fetch(chain0 + step, stages + ((k & 1) ^ 1) * 3 * NC * kSet);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      for (int q = tid; q < NC * DD; q += 32 * kGradWarps) {
+        const int sub = q / DD, e = q % DD;
+        if (chain0 + sub >= chains) break;
+        int a, ab, row, col;
+        chain_pair(chain0 + sub, a, ab);
+        order_rc<DB>(e, row, col);
+        const double2 *B = stage + sub * 3 * kSet + e, *S = B + kSet, *R = S + kSet;
+        double2 *V = ops + sub * 2 * kSet + e, *O = V + kSet;
+        const double2 zero = make_double2(0.0, 0.0);
+        auto scaled = [](double f, double2 x) { return make_double2(f * x.x, f * x.y); };
+        auto plus = [](double2 x, double2 y) { return make_double2(x.x + y.x, x.y + y.y); };
+        int bra = last_bit(col, nb), ket = last_bit(row, nb);
+        if (first) {
+          const int b0 = bra ^ last_bit(ab, nb), k0 = ket ^ last_bit(a, nb);
+          const double2 v = cmul_conj(T0[frag_at<DB>(row, a)], T0[frag_at<DB>(col, ab)]);
+          const double2 zv = scaled(-m_z(m1, b0, k0), v);
+          V[kI * DD] = b0 == k0 ? v : zero;
+          V[kX * DD] = cmul(m_x(m1, b0, k0), v);
+          V[kH * DD] = zv;
+          V[kW * DD] = zero;
+          V[kS * DD] = zv;
         } else {
-          const bool first = w - 1 == 1;
-          const int src = c == kX ? kI : (c == kW && first ? kX : c);
-          v = load_mat<DB>(before + src * DD, lane);
-          if (c == kX || (c == kW && first)) {
-            each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-              const double2 x = cmul(m_x(m1, bra, ket), make_double2(v.re[i][j][e], v.im[i][j][e]));
-              v.re[i][j][e] = x.x;
-              v.im[i][j][e] = x.y;
-            });
-          } else if (c == kS && !first) {
-            each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-              const double z = m_z(m1, bra, ket);
-              v.re[i][j][e] *= z;
-              v.im[i][j][e] *= z;
-            });
-          } else {
-            each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-              if (bra != ket) v.re[i][j][e] = v.im[i][j][e] = 0.0;
-            });
-            if (c == kH)
-              each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-                const int at = (i * DB + j) * 64 + 2 * lane + e;
-                const double2 x = cmul(m_x(m1, bra, ket), before[kX * DD + at]);
-                const double z = first ? 0.0 : m_z(m1, bra, ket);
-                const double2 ti = before[kI * DD + at];
-                v.re[i][j][e] += -z * ti.x - h * x.x;
-                v.im[i][j][e] += -z * ti.y - h * x.y;
-              });
-          }
+          const double2 x1 = m_x(m1, bra, ket), tI = B[kI * DD], tX = cmul(x1, B[kX * DD]);
+          const double z1 = m_z(m1, bra, ket);
+          double2 hh = scaled(-h, tX);
+          if (!second) hh = plus(hh, scaled(-z1, tI));
+          if (bra == ket) hh = plus(hh, B[kH * DD]);
+          V[kI * DD] = bra == ket ? tI : zero;
+          V[kX * DD] = cmul(x1, tI);
+          V[kH * DD] = hh;
+          V[kW * DD] = second ? tX : (bra == ket ? B[kW * DD] : zero);
+          V[kS * DD] = second ? (bra == ket ? B[kS * DD] : zero) : scaled(z1, B[kS * DD]);
         }
-        // right component behind the site's last layer, and that layer's sums
-        Mat<DB> r = zero_mat<DB>(), q = zero_mat<DB>();
-        if (w < n - 1 && (c == kI || c == kS || c == kW)) {
-          if (c != kW || w > 1) r = right_of(c, chain);
-        }
-        if (c == kS && w == n - 1) r = rH;
-        Mat<DB> rW1;
-        if (c == kX && w == 1) rW1 = right_of(kW, chain);
-        if (c != kH) q = load_mat<DB>(here + c * DD, lane);
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int bra, int ket) {
-          const double2 H = make_double2(rH.re[i][j][e], rH.im[i][j][e]);
-          const double2 X = make_double2(rX.re[i][j][e], rX.im[i][j][e]);
-          const double2 mx = m_x(m, bra, ket);
-          const double z = m_z(m, bra, ket);
-          const double2 tq = make_double2(q.re[i][j][e], q.im[i][j][e]);
-          double2 o = make_double2(r.re[i][j][e], r.im[i][j][e]);
-          if (c == kI) {
-            const double zz = w == 1 ? 0.0 : z;
-            const double2 x = cmul(mx, X);
-            last_layer(bra, ket, cmul(tq, X),
-                       w == 1 ? make_double2(0.0, 0.0) : cmul(tq, make_double2(-H.x, -H.y)));
-            if (bra != ket) o = make_double2(0.0, 0.0);
-            o.x += x.x - zz * H.x;
-            o.y += x.y - zz * H.y;
-          } else if (c == kX || (c == kW && w == n - 1)) {
-            double2 x = make_double2(-h * H.x, -h * H.y);
-            if (c == kX && w == 1) {
-              x.x += rW1.re[i][j][e];
-              x.y += rW1.im[i][j][e];
-            }
-            last_layer(bra, ket, cmul(tq, x), make_double2(0.0, 0.0));
-            o = cmul(mx, x);
-          } else if (c == kH) {
-            o = bra == ket ? H : make_double2(0.0, 0.0);
-          } else if (c == kW || w == 1) {
-            if (bra != ket) o = make_double2(0.0, 0.0);
-          } else {
-            last_layer(bra, ket, make_double2(0.0, 0.0), cmul(tq, o));
-            o = make_double2(z * o.x, z * o.y);
-          }
-          r.re[i][j][e] = o.x;
-          r.im[i][j][e] = o.y;
-        });
-        // y[s'][bra] = sum v[s'][.] conj(T[bra][.]); g[s][s'] += sum r[s][bra] y[s'][bra]
-        Mat<DB> vc = v;
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int, int) { vc.im[i][j][e] = -vc.im[i][j][e]; });
-        Mat<DB> y = zero_mat<DB>();
-        mma_rows<DB, false>(y, vc, t);  // conj(v) T: the conjugate of y
-        each<DB>(lane, nb, 0, 0, [&](int i, int j, int e, int, int) { y.im[i][j][e] = -y.im[i][j][e]; });
-        mma_rows<DB, false>(g, r, y);
+        const double2 x = m_x(m, bra, ket);
+        const double z = m_z(m, bra, ket);
+        const double2 one = make_double2(row == a && col == ab ? 1.0 : 0.0, 0.0);
+        const double2 rI = end ? zero : R[kI * DD], rX = end ? zero : R[kX * DD], rH = end ? one : R[kH * DD];
+        const double2 rW = end ? zero : R[kW * DD], rS = end ? one : R[kS * DD];
+        const double2 hH = scaled(-h, rH);
+        double2 o = cmul(x, rX);
+        if (bra == ket) o = plus(o, rI);
+        O[kI * DD] = first ? o : plus(o, scaled(-z, rH));
+        const double2 xx = first ? plus(hH, rW) : hH;
+        O[kX * DD] = cmul(x, xx);
+        O[kH * DD] = bra == ket ? rH : zero;
+        O[kW * DD] = end ? cmul(x, hH) : (first || bra != ket ? zero : rW);
+        O[kS * DD] = first ? (bra == ket ? rS : zero) : scaled(z, rS);
+        // the last layer's sums; the mirrored pair's are their conjugates
+        double2 qx = plus(cmul(S[kI * DD], rX), cmul(S[kX * DD], xx));
+        if (end) qx = plus(qx, cmul(S[kW * DD], hH));
+        const double twice = a == ab ? 1.0 : 2.0;
+        const double2 xt = m_x(mt, bra, ket), xp = m_x(mp, bra, ket);
+        double dt = xt.x * qx.x - xt.y * qx.y;
+        if (!first) dt += m_z(mt, bra, ket) * (cmul(S[kS * DD], rS).x - cmul(S[kI * DD], rH).x);
+        g_theta += twice * dt;
+        g_phi += twice * (xp.x * qx.x - xp.y * qx.y);
       }
+      __syncthreads();
+      const Mat<DB, DB> t = load_mat<DB>(T, lane);
+#pragma unroll 1
+      for (int sub = 0; sub < NC && chain0 + sub < chains; ++sub) {
+        int a, ab;
+        chain_pair(chain0 + sub, a, ab);
+        const double2 *V = ops + sub * 2 * kSet + c * DD, *O = V + kSet;
+#pragma unroll 1
+        for (int mirror = DB == 1 ? warp % 2 : 0; mirror < (a == ab ? 1 : 2); mirror += DB == 1 ? 2 : 1) {
+          const Mat<1, DB> v = load_rows<DB, 1>(V, mirror != 0, js, true, lane);
+          Mat<1, DB> y = zero_mat<1, DB>();
+          mma_rows<false, false, false, false>(y, v, t);  // conj(V) T: the conjugate of y
+          elements<1, DB>([&](int i, int j, int e) { y.im[i][j][e] = -y.im[i][j][e]; });
+          const Mat<DB, DB> r = load_rows<DB, DB>(O, mirror != 0, 0, false, lane);
+          // (an identity's R: at L = 5 its off-diagonal tiles are zero)
+          if (DB > 1 && (c == kH || (c == kW && !end))) mma_rows<false, false, false, true>(g, r, y);
+          else mma_rows<false, false, false, false>(g, r, y);
+        }
+      }
+      __syncthreads();  // the operands are read
     }
-    store_mat<DB>(G + warp * DD, g, lane);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    elements<DB, 1>([&](int i, int, int e) {
+      G[(warp / DB) * DD + (i * DB + js) * 64 + 32 * e + lane] = make_double2(g.re[i][0][e], g.im[i][0][e]);
+    });
   }
   __syncthreads();
   // The site's derivatives from dE/dT = 2 Re sum G dT (linear: every CTA its part)
@@ -651,7 +702,7 @@ __global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingPa
   for (int e = tid; e < DD; e += 32 * kGradWarps) {
     double2 g = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int k = 0; k < kGradWarps; ++k) {
+    for (int k = 0; k < kSlices; ++k) {
       g.x += G[k * DD + e].x;
       g.y += G[k * DD + e].y;
     }
@@ -697,22 +748,29 @@ __global__ void __launch_bounds__(32 * kGradWarps) ring_grad_kernel(const RingPa
     if (lane == 0) red[warp][k] = s;
   }
   __syncthreads();
+  // this CTA's part; the site's last CTA to finish adds them in order
+  double *parts = P.grad_parts + static_cast<size_t>(w) * G_ctas * kMaxDerivs;
   if (tid < kMaxDerivs) {
     double s = 0.0;
 #pragma unroll
     for (int k = 0; k < kGradWarps; ++k) s += red[k][tid];
-    total[tid] = s;
+    parts[rank * kMaxDerivs + tid] = s;
+    __threadfence();
   }
-  cluster.sync();
-  if (rank == 0 && tid < 2 * L) {
+  __shared__ bool last;
+  __syncthreads();
+  if (tid == 0)
+    last = atomicInc(P.counter + 1 + w, static_cast<unsigned>(G_ctas - 1)) == static_cast<unsigned>(G_ctas - 1);
+  __syncthreads();
+  if (last && tid < 2 * L) {
+    __threadfence();
     double s = 0.0;
-    for (int k = 0; k < G_ctas; ++k) s += *cluster.map_shared_rank(total + tid, k);
+    for (int k = 0; k < G_ctas; ++k) s += __ldcg(parts + k * kMaxDerivs + tid);
     // a NaN energy (a non-finite angle) voids the whole gradient
     const double energy = P.energy_parts[chains];
     if (energy != energy) s = energy;
     P.grad_out[static_cast<size_t>(tid / 2 * n + w) * 2 + (tid & 1)] = s;
   }
-  cluster.sync();  // peers' shared memory stays until it is read
 }
 
 template <int DB>
@@ -729,21 +787,25 @@ cudaError_t sweeps(const RingParams &P, int first, int dirs, bool keep, cudaStre
 template <int DB>
 cudaError_t gradient(const RingParams &P, cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  constexpr size_t smem = sizeof(double2) * (2 + kGradWarps) * 64 * DB * DB;
+  constexpr size_t smem = sizeof(double2) * (2 + kGradWarps / DB + 8 * chains_a_step<DB>() * kComps) * 64 * DB * DB;
   cudaError_t e = set_smem_limit_once(ring_grad_kernel<DB>, smem, done);
   if (e != cudaSuccess) return e;
-  // two chains a warp, four CTAs a site at 64 chains, at most eight
-  int ctas = 1;
-  while (ctas < 8 && ctas * 2 * kGradWarps < ring_chains(P.L)) ctas *= 2;
+  // at most eight CTAs a site, no more than its chains need, and no more (one CTA
+  // an SM) than fill the SMs once
+  const int steps = (ring_chains(P.L) + chains_a_step<DB>() - 1) / chains_a_step<DB>();
+  int ctas = steps < 8 ? steps : 8;
+  int dev = 0, sms = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  while (ctas > 1 && ctas * P.n > sms) --ctas;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(P.n * ctas));
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(P.n));
   cfg.blockDim = dim3(32 * kGradWarps);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = static_cast<unsigned>(ctas);
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, ring_grad_kernel<DB>, P);

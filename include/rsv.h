@@ -76,10 +76,12 @@ const char *rsv_stage_name(int i);
  * does and otherwise ignored (the engine plans its own tiles).
  * Allocates three state buffers of 16 * 2^max(n,12) bytes.
  * A structured_adjoint circuit of few layers is contracted along the ring
- * (gpu_simulation_b200/csrc/rsv_ring.cu) instead of running the tile passes,
- * with the same results to rounding, as long as the backward schedule, the
- * analytic layers and the kernel flags below are at their defaults; setting
- * one of them otherwise selects the tile passes.
+ * (gpu_simulation_b200/csrc/rsv_ring.cu), another one of up to 16 qubits and
+ * 64 layers keeps its state in one thread-block cluster (rsv_cluster.cu),
+ * instead of running the tile passes, with the same results to rounding, as
+ * long as the backward schedule, the analytic layers and the kernel flags
+ * below are at their defaults; setting one of them otherwise selects the tile
+ * passes.
  */
 rsv_status rsv_create(int num_qubits, int num_layers, double field,
                       const char *gradient_strategy, int structured_rotation_chunk_width,
