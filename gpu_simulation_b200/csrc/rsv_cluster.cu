@@ -35,6 +35,13 @@
 // sum_i z_w(i) Im(conj(lambda_i) psi_i).
 //
 // Sums go through fixed orders (lanes, warps, CTAs): equal inputs give equal bits.
+//
+// Bound by latency up to 12 qubits (one launch against one a layer and pass:
+// energy and gradient at L = 8, n = 8 246 -> 18.7 us, n = 10 256 -> 31, n = 12
+// 269 -> 64) and by the stores into other CTAs above (about 9 to 12 bytes a clock
+// and SM; n = 14 327 -> 120 us, n = 16 336 -> 293).  Every shape is its own
+// instantiation: with the layouts' arithmetic at run time n = 8 took 58 us and
+// n = 12 118, most of it integer and address latency.
 #include <cuda_runtime.h>
 
 #include <atomic>

@@ -6,17 +6,27 @@
 
 namespace rsv {
 
-// C[m][n] = sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] (+ bias[n]); Z (if not
-// null) receives the pre-activation, C the GELU of it when gelu_act.
-cudaError_t mlp_gemm(int M, int N, int K, const float *A, long long sam, long long sak,
-                     const float *B, long long sbk, long long sbn, const float *bias, bool gelu_act,
-                     float *C, float *Z, cudaStream_t s);
-cudaError_t mlp_gelu_back(long long count, const float *Z, const float *dY, float *dZ,
-                          cudaStream_t s);
-cudaError_t mlp_colsum(int M, int N, const float *dZ, float *db, cudaStream_t s);
-int mlp_loss_blocks(long long count);
-cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout,
-                    float *partials, float *loss, cudaStream_t s);
+// One product C[m][n] = sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] (C is M x N,
+// row-major) and what follows it: + bias[n], the sum itself to Z, GELU, times
+// GELU's derivative at gelu_of[m][n] (each where not null / set).  row_sums[m]
+// receives sum_k A(m, k) where not null.
+struct MlpGemm {
+  int M, N, K;
+  const float *A;
+  long long sam, sak;
+  const float *B;
+  long long sbk, sbn;
+  float *C;
+  const float *bias;
+  float *Z;
+  const float *gelu_of;
+  float *row_sums;
+  bool gelu;
+};
+// One or two independent products in one launch.
+cudaError_t mlp_gemm(const MlpGemm *g, int count, cudaStream_t s);
+cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout, float *loss,
+                    cudaStream_t s);
 cudaError_t gd_step(long long count, double *p, const double *g, double stepsize, const double *energy,
                     double *energy_hist, double *gnorm_hist, int *counter, cudaStream_t s);
 cudaError_t adam_vqe_step(long long count, double *p, const double *g, double *m, double *v, double lr,

@@ -107,7 +107,21 @@ rsv_status rsv_mlp_forward(int num_layers, const int *widths, const float *d_wei
       const bool hidden = l < num_layers;
       float *Z = hidden ? work : nullptr;
       float *A = hidden ? work + static_cast<size_t>(batch) * N : d_out;
-      cuda_check(mlp_gemm(batch, N, K, x, K, 1, W, 1, K, b, hidden, A, Z, s), "mlp forward gemm");
+      MlpGemm g{};
+      g.M = batch;
+      g.N = N;
+      g.K = K;
+      g.A = x;
+      g.sam = K;
+      g.sak = 1;
+      g.B = W;
+      g.sbk = 1;
+      g.sbn = K;
+      g.C = A;
+      g.bias = b;
+      g.Z = Z;
+      g.gelu = hidden;
+      cuda_check(mlp_gemm(&g, 1, s), "mlp forward gemm");
       if (hidden) work += 2 * static_cast<size_t>(batch) * N;
       x = A;
     }
@@ -142,18 +156,37 @@ rsv_status rsv_mlp_backward(int num_layers, const int *widths, const float *d_we
       float *gW = d_grad + woff[l], *gb = gW + static_cast<size_t>(N) * K;
       // input of layer l: the network input, or the post-activation of layer l-1
       const float *X = (l == 1) ? d_x : d_work + aoff[l - 1] + static_cast<size_t>(batch) * K;
-      // dW = dZ^T X  (N x K, summed over the batch)
-      cuda_check(mlp_gemm(N, K, batch, dZ, 1, N, X, K, 1, nullptr, false, gW, nullptr, s),
-                 "mlp weight-gradient gemm");
-      cuda_check(mlp_colsum(batch, N, dZ, gb, s), "mlp bias gradient");
+      // dW = dZ^T X  (N x K, summed over the batch), db = its first operand's row sums
+      MlpGemm g[2] = {};
+      g[0].M = N;
+      g[0].N = K;
+      g[0].K = batch;
+      g[0].A = dZ;
+      g[0].sam = 1;
+      g[0].sak = N;
+      g[0].B = X;
+      g[0].sbk = K;
+      g[0].sbn = 1;
+      g[0].C = gW;
+      g[0].row_sums = gb;
+      float *dA = nullptr;
       if (l > 1) {
-        float *dA = bufs[l & 1];
-        // dA = dZ W  (batch x K), then dZ_{l-1} = dA * gelu'(Z_{l-1}) in place
-        cuda_check(mlp_gemm(batch, K, N, dZ, N, 1, W, K, 1, nullptr, false, dA, nullptr, s),
-                   "mlp input-gradient gemm");
-        const float *Zprev = d_work + aoff[l - 1];
-        cuda_check(mlp_gelu_back(static_cast<long long>(batch) * K, Zprev, dA, dA, s),
-                   "mlp gelu backward");
+        dA = bufs[l & 1];
+        // dZ_{l-1} = (dZ W) * gelu'(Z_{l-1})  (batch x K)
+        g[1].M = batch;
+        g[1].N = K;
+        g[1].K = N;
+        g[1].A = dZ;
+        g[1].sam = N;
+        g[1].sak = 1;
+        g[1].B = W;
+        g[1].sbk = K;
+        g[1].sbn = 1;
+        g[1].C = dA;
+        g[1].gelu_of = d_work + aoff[l - 1];
+      }
+      cuda_check(mlp_gemm(g, l > 1 ? 2 : 1, s), "mlp backward gemms");
+      if (l > 1) {
         dZ = dA;
       }
     }
@@ -165,7 +198,7 @@ rsv_status rsv_mlp_mse(size_t count, const float *d_out, const float *d_target, 
   return mlp_guarded([&] {
     if (count == 0) throw ArgError("count must be positive");
     if (!d_out || !d_target || !d_dout || !d_loss || !d_partials) throw ArgError("null device pointer");
-    cuda_check(mlp_mse(static_cast<long long>(count), d_out, d_target, d_dout, d_partials, d_loss,
+    cuda_check(mlp_mse(static_cast<long long>(count), d_out, d_target, d_dout, d_loss,
                        static_cast<cudaStream_t>(stream)),
                "mse");
   });

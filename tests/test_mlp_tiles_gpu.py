@@ -1,0 +1,33 @@
+"""The network's products at the edges of their 32 x 32 tiles, of the four-way
+depth split and of its 16-deep stages, against the float64 oracle."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import mlp
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("widths,batch", [
+    ((1, 1), 1), ((16, 32, 64), 31), ((65, 33, 1), 64), ((63, 64, 96), 129), ((128, 31, 33), 257), ((4, 8, 4), 1000),
+])
+def test_loss_and_gradient_match_oracle(widths, batch):
+    import torch
+
+    from gpu_simulation_b200.warmstart import WarmStartMLP
+
+    net = WarmStartMLP(widths, seed=5)
+    rng = np.random.default_rng(6)
+    x = rng.uniform(-1.0, 2.0, (batch, widths[0])).astype(np.float32)
+    t = rng.uniform(-3.0, 3.0, (batch, widths[-1])).astype(np.float32)
+    loss, grad = net.gradient(torch.from_numpy(x), torch.from_numpy(t))
+    w64 = net.weights.cpu().numpy().astype(np.float64)
+    out, cache = mlp.forward(w64, widths, x.astype(np.float64))
+    l_ref, dout = mlp.mse(out, t.astype(np.float64))
+    g_ref = mlp.backward(w64, widths, cache, dout)
+    # float32 sums of at most 1000 terms: sqrt(1000) * 6e-8 of the largest entry, with room
+    assert abs(loss.item() - l_ref) < 1e-5 * abs(l_ref)
+    np.testing.assert_allclose(grad.cpu().numpy(), g_ref, atol=1e-5 * np.abs(g_ref).max(), rtol=1e-3)
