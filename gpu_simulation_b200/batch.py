@@ -155,6 +155,11 @@ class BatchEngine:
     def set_active_slots(self, slots: int) -> None:
         check(self._lib.rsv_batch_set_active_slots(self._h, int(slots)))
 
+    def set_resident(self, resident: bool = True) -> None:
+        """Cluster-resident circuits (the default) or the persistent kernel,
+        which set_active_slots and set_cluster also choose."""
+        check(self._lib.rsv_batch_set_resident(self._h, int(bool(resident))))
+
     def set_cluster(self, cluster: int) -> None:
         """CTAs per thread-block cluster (1, 2, 4 or 8): a large circuit is
         spread over up to this many SMs, and the cluster's CTAs add their
@@ -221,16 +226,17 @@ class BatchEngine:
         return graph
 
     def autotune(self, params, energy_out, grad_out=None, candidates=None, repeats: int = 3) -> dict:
-        """Time the batch for each cluster size (1, 2, 4, 8 CTAs) and a few
-        numbers of CTAs in flight, and keep the fastest (bigger clusters spread
-        large circuits over more SMs and keep fewer of them, and their states,
-        in flight; more CTAs keep every SM busy).  Returns
-        {"cluster x CTAs": ms} and sets the best."""
+        """Time the batch cluster-resident and on the persistent kernel for each
+        cluster size (1, 2, 4, 8 CTAs) and a few numbers of CTAs in flight, and
+        keep the fastest (bigger clusters spread large circuits over more SMs
+        and keep fewer of them, and their states, in flight; more CTAs keep
+        every SM busy).  Given candidates (cluster, CTAs) stand for themselves.
+        Returns {"resident" or "cluster x CTAs": ms} and sets the best."""
         import torch
 
         full = self.max_slots
         if candidates is None:
-            candidates = []
+            candidates = ["resident"]
             for c in (1, 2, 4, 8):
                 if c > full:
                     continue
@@ -239,20 +245,25 @@ class BatchEngine:
         times = {}
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
-        for c, k in candidates:
+        for cand in candidates:
             try:
-                self.set_cluster(c)
-            except ValueError:
+                self._apply(cand)
+            except (ValueError, RuntimeError):
                 continue  # no cluster of this size fits
-            self.set_active_slots(k)
             self.run_device(params, energy_out, grad_out)
             a.record()
             for _ in range(repeats):
                 self.run_device(params, energy_out, grad_out)
             b.record()
             b.synchronize()
-            times[(c, int(k))] = a.elapsed_time(b) / repeats
+            times[cand] = a.elapsed_time(b) / repeats
         best = min(times, key=times.get)
-        self.set_cluster(best[0])
-        self.set_active_slots(best[1])
-        return {f"{c}x{k}": ms for (c, k), ms in times.items()}
+        self._apply(best)
+        return {c if c == "resident" else f"{c[0]}x{int(c[1])}": ms for c, ms in times.items()}
+
+    def _apply(self, candidate) -> None:
+        if candidate == "resident":
+            self.set_resident(True)
+        else:
+            self.set_cluster(candidate[0])
+            self.set_active_slots(candidate[1])

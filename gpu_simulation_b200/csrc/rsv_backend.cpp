@@ -1529,6 +1529,19 @@ struct rsv_batch {
   rsv::DevBuf<rsv::BatchGroup> d_groups;
   rsv::DevBuf<int> d_counter;
   cudaStream_t stream = nullptr;
+  // Cluster-resident circuits (rsv_cluster.cu), the default: one launch per
+  // qubit count, largest first, on streams forked from the caller's.  A caller
+  // that gave slots, or set them or a cluster size, chose the persistent kernel.
+  bool resident = true;
+  struct Class {
+    int n, first, count, max_layers;
+  };
+  std::vector<Class> classes;
+  unsigned int fits = 0;  // qubit counts whose clusters fit the device
+  rsv::DevBuf<rsv::ClusterItem> d_items;
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> joined;
+  cudaEvent_t forked = nullptr;
 };
 
 namespace rsv {
@@ -1609,6 +1622,65 @@ void batch_group(rsv_batch *Bt) {
   Bt->num_groups = static_cast<int>(groups.size());
 }
 
+// How a batch spreads its circuits, for throughput: 16 amplitudes a thread from
+// 10 qubits on, as few CTAs as hold the state (4096 amplitudes each).  At L = 8
+// and as many CTAs as an SM holds: n = 9 5 us a circuit and SM (16 a thread 5.9),
+// n = 10 10.8 (8 a thread 15.5), n = 11 25 (49), n = 12 90.
+ClusterShape batch_shape_for(int n) {
+  if (n <= 8) return {0, 2};
+  if (n == 9) return {0, 3};
+  return {std::max(0, n - kTileBits), 4};
+}
+
+// The circuits by qubit count (largest first) and depth (deepest first); false
+// where the device does not hold a cluster of some class.
+bool batch_classes(rsv_batch *Bt, const std::vector<BatchCircuit> &circ) {
+  std::vector<int> order(circ.size());
+  for (size_t c = 0; c < circ.size(); ++c) order[c] = static_cast<int>(c);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    const BatchCircuit &x = circ[static_cast<size_t>(a)], &y = circ[static_cast<size_t>(b)];
+    return x.n != y.n ? x.n > y.n : x.L > y.L;
+  });
+  std::vector<ClusterItem> items;
+  Bt->classes.clear();
+  for (int c : order) {
+    const BatchCircuit &C = circ[static_cast<size_t>(c)];
+    if (Bt->classes.empty() || Bt->classes.back().n != C.n) {
+      if (!((Bt->fits >> C.n) & 1)) {  // asked once a qubit count, for the deepest circuits
+        int clusters = 0;
+        check(cluster_capacity(C.n, batch_shape_for(C.n), kBatchMaxLayers, &clusters), "cluster capacity");
+        if (clusters < 1) return false;
+        Bt->fits |= 1u << C.n;
+      }
+      Bt->classes.push_back({C.n, static_cast<int>(items.size()), 0, C.L});
+    }
+    ++Bt->classes.back().count;
+    ClusterItem it{};
+    it.L = C.L;
+    it.index = C.index;
+    it.param_off = C.param_off;
+    it.h = C.h;
+    items.push_back(it);
+  }
+  while (Bt->side.size() + 1 < Bt->classes.size()) {
+    // the larger circuits' clusters go first where both wait for SMs
+    int least = 0, greatest = 0;
+    check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream priorities");
+    const int level = std::min(least, greatest + 1 + static_cast<int>(Bt->side.size()));
+    cudaStream_t s = nullptr;
+    check(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, level), "cudaStreamCreate");
+    Bt->side.push_back(s);
+    cudaEvent_t e = nullptr;
+    check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    Bt->joined.push_back(e);
+  }
+  if (Bt->forked == nullptr)
+    check(cudaEventCreateWithFlags(&Bt->forked, cudaEventDisableTiming), "cudaEventCreate");
+  upload(Bt->d_items, items, Bt->stream, "batch item upload");
+  check(cudaStreamSynchronize(Bt->stream), "batch upload");
+  return true;
+}
+
 void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, const double *hs) {
   if (count < 0) invalid("count must be non-negative");
   if (count > 0 && (ns == nullptr || Ls == nullptr || hs == nullptr)) invalid("null circuit array");
@@ -1635,6 +1707,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
         Bt->plan_cost[static_cast<size_t>(C.plan)] * static_cast<double>(u64{1} << std::max(n, kTileBits));
     off += static_cast<size_t>(2) * n * L;
   }
+  if (Bt->resident && count > 0 && !batch_classes(Bt, circ)) Bt->resident = false;
   cudaStream_t st = Bt->stream;
   if (Bt->dirty) {
     upload(Bt->d_plans, Bt->plans, st, "batch plan upload");
@@ -1655,6 +1728,33 @@ void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *
                cudaStream_t st) {
   if (Bt->count == 0) return;
   if (d_params == nullptr || d_energy == nullptr) invalid("null device pointer");
+  if (Bt->resident) {
+    auto launch = [&](const rsv_batch::Class &c, cudaStream_t s) {
+      ClusterArgs A{};
+      const ClusterShape h = batch_shape_for(c.n);
+      A.n = c.n;
+      A.log_ctas = h.log_ctas;
+      A.register_bits = h.register_bits;
+      A.count = c.count;
+      A.items = Bt->d_items.p + c.first;
+      A.max_layers = c.max_layers;
+      A.params = d_params;
+      A.energy_out = d_energy;
+      A.grad_out = d_grad;
+      check(launch_cluster(A, s), "batch launch");
+    };
+    const size_t others = Bt->classes.size() - 1;
+    if (others > 0) check(cudaEventRecord(Bt->forked, st), "cudaEventRecord");
+    launch(Bt->classes[0], st);
+    for (size_t k = 0; k < others; ++k) {
+      check(cudaStreamWaitEvent(Bt->side[k], Bt->forked, 0), "cudaStreamWaitEvent");
+      launch(Bt->classes[k + 1], Bt->side[k]);
+      check(cudaEventRecord(Bt->joined[k], Bt->side[k]), "cudaEventRecord");
+    }
+    for (size_t k = 0; k < others; ++k)
+      check(cudaStreamWaitEvent(st, Bt->joined[k], 0), "cudaStreamWaitEvent");
+    return;
+  }
   BatchArgs A{};
   A.count = Bt->count;
   A.circuits = Bt->d_circuits.p;
@@ -2685,6 +2785,7 @@ rsv_status rsv_batch_create(int max_qubits, int slots, rsv_batch **out) {
     Bt->max_qubits = max_qubits;
     Bt->slots = slots > 0 ? slots : Bt->sms;
     Bt->active_slots = Bt->slots;
+    Bt->resident = slots == 0;
     // the largest cluster (8, 4, 2, 1) that the slots and the device hold
     Bt->cluster = 8;
     while (Bt->cluster > 1 && (Bt->cluster > Bt->slots || batch_max_active_clusters(Bt->cluster) < 1))
@@ -2704,6 +2805,9 @@ rsv_status rsv_batch_destroy(rsv_batch *batch) {
     if (batch == nullptr) return;
     cudaStreamSynchronize(batch->stream);
     cudaStreamDestroy(batch->stream);
+    for (auto s : batch->side) cudaStreamDestroy(s);
+    for (auto e : batch->joined) cudaEventDestroy(e);
+    if (batch->forked) cudaEventDestroy(batch->forked);
     delete batch;
   });
 }
@@ -2735,6 +2839,7 @@ rsv_status rsv_batch_set_active_slots(rsv_batch *batch, int slots) {
     if (slots < 1 || slots > batch->slots)
       invalid("slots must be in [1, " + std::to_string(batch->slots) + "]");
     batch->active_slots = slots;
+    batch->resident = false;
   });
 }
 
@@ -2747,7 +2852,20 @@ rsv_status rsv_batch_set_cluster(rsv_batch *batch, int cluster) {
     if (batch_max_active_clusters(cluster) < 1) invalid("no cluster of this size fits on the device");
     check(cudaStreamSynchronize(batch->stream), "batch synchronize");
     batch->cluster = cluster;
+    batch->resident = false;
     batch_group(batch);
+  });
+}
+
+rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident) {
+  return guarded([&] {
+    const OnDevice on_device(batch ? batch->device : -1);
+    if (batch == nullptr) invalid("batch is null");
+    batch->resident = resident != 0;
+    if (batch->resident && batch->count > 0 && !batch_classes(batch, batch->circuits)) {
+      batch->resident = false;
+      throw Error(RSV_ERR_UNSUPPORTED, "a cluster of these circuits does not fit the device");
+    }
   });
 }
 

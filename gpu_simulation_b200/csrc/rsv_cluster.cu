@@ -737,12 +737,19 @@ bool with_shape(int n, ClusterShape h, F &&f) {
   one(Shape<7, 2, 0>{});
   one(Shape<8, 2, 0>{});
   one(Shape<9, 2, 0>{});
+  one(Shape<9, 3, 0>{});
   one(Shape<10, 3, 0>{});
+  one(Shape<10, 4, 0>{});
   one(Shape<11, 3, 0>{});
+  one(Shape<11, 4, 0>{});
   one(Shape<12, 3, 3>{});
+  one(Shape<12, 4, 0>{});
   one(Shape<13, 3, 3>{});
+  one(Shape<13, 4, 1>{});
   one(Shape<14, 4, 4>{});
+  one(Shape<14, 4, 2>{});
   one(Shape<15, 4, 4>{});
+  one(Shape<15, 4, 3>{});
   one(Shape<16, 4, 4>{});
   return found;
 }

@@ -334,8 +334,11 @@ unsigned long long rsv_ring_map(unsigned long long index, int num_qubits, int in
 /*
  * Batched circuits: many independent ring-Ising circuits of uneven size
  * (2 <= num_qubits <= RSV_BATCH_MAX_QUBITS, 1 <= num_layers <=
- * RSV_BATCH_MAX_LAYERS, own field each) evaluated by ONE persistent kernel
- * launch.  No counterpart in the reference, which evaluates one circuit per
+ * RSV_BATCH_MAX_LAYERS, own field each) evaluated by one launch per qubit
+ * count, every circuit's state resident in the registers and shared memory of
+ * one thread-block cluster (the default), or by ONE persistent kernel whose
+ * states stream through scratch slots (chosen by giving slots at creation, by
+ * rsv_batch_set_active_slots or by rsv_batch_set_cluster).  No counterpart in the reference, which evaluates one circuit per
  * backend object; a batch of circuits there is a loop over
  * RingIsingCudaBackend::energy_and_grad (reference cpp/ising_cuda_backend.hpp:38-41).
  *
@@ -346,9 +349,10 @@ unsigned long long rsv_ring_map(unsigned long long index, int num_qubits, int in
  * rsv_batch_set_circuits builds (or reuses) the pass plan of every distinct
  * (num_qubits, num_layers), sorts the circuits by decreasing cost and uploads
  * the descriptors; it is synchronous.  rsv_batch_run_device enqueues the
- * whole batch on `stream` (used as given; 0 = legacy default stream): a
- * counter reset and one kernel launch, no allocation and no host
- * synchronisation, so it can be captured into a CUDA graph.  d_gradient_out
+ * whole batch on `stream` (used as given; 0 = legacy default stream), with
+ * the launches of further qubit counts on streams forked from it and joined to
+ * it again: no allocation and no host synchronisation, so it can be captured
+ * into a CUDA graph.  d_gradient_out
  * NULL computes energies only.  A handle is not re-entrant.
  */
 #define RSV_BATCH_MAX_QUBITS 16
@@ -367,6 +371,10 @@ rsv_status rsv_batch_set_circuits(rsv_batch *batch, int count, const int *num_qu
 /* Circuits and packed parameter count of the current description. */
 rsv_status rsv_batch_info(rsv_batch *batch, int *count, size_t *num_params, int *slots,
                           size_t *device_bytes);
+
+/* Run the following batches cluster-resident (non-zero) or on the persistent
+ * kernel. */
+rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident);
 
 /* CTAs in flight for the following runs (1..the slots given at creation;
  * rounded down to whole clusters); used by the autotuner
