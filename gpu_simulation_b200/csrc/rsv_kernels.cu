@@ -105,6 +105,8 @@ __global__ void tables_kernel(const double4 *__restrict__ coef, int n, int L,
 __global__ void rot_kernel(const double4 *__restrict__ coef, int n, int L, const int *__restrict__ order,
                            int checkpoint, double2 *__restrict__ rot, double *__restrict__ lscale,
                            double *__restrict__ gscale) {
+  __shared__ double factors[kMaxQubits];
+  __shared__ int wires[kMaxQubits];  // the layer's undo order
   const int layer = blockIdx.x;
   if (layer >= L) return;
   order += layer * n;
@@ -112,21 +114,23 @@ __global__ void rot_kernel(const double4 *__restrict__ coef, int n, int L, const
     const double4 k = coef[layer * n + w];
     rot[layer * n + w] = (fabs(k.x) >= fabs(k.y)) ? make_double2(k.y / k.x, 1.0)
                                                    : make_double2(k.x / k.y, -1.0);
+    factors[w] = (fabs(k.x) >= fabs(k.y)) ? k.x : k.y;
+    wires[w] = order[w];
   }
+  __syncthreads();
   if (threadIdx.x != 0) return;
-  auto factor = [&](int w) {
-    const double4 k = coef[layer * n + w];
-    return (fabs(k.x) >= fabs(k.y)) ? k.x : k.y;
-  };
+  order = wires;
+  auto factor = [&](int w) { return factors[w]; };
   double K = 1.0;
   for (int w = 0; w < n; ++w) K *= factor(w);
   lscale[layer] = K;
+  const double phi_scale = 1.0 / (K * K);
   if (!checkpoint) {
     double pending = K;
     for (int i = 0; i < n; ++i) {
       const int w = order[i] & (kUndoPassStart - 1);
       gscale[2 * (layer * n + w)] = 1.0 / (pending * pending);
-      gscale[2 * (layer * n + w) + 1] = 1.0 / (K * K);
+      gscale[2 * (layer * n + w) + 1] = phi_scale;
       pending /= factor(w);
     }
   } else {
@@ -148,7 +152,7 @@ __global__ void rot_kernel(const double4 *__restrict__ coef, int n, int L, const
         group = 1.0;
       }
       gscale[2 * (layer * n + w)] = undone * undone / (first ? K * K : 1.0);
-      gscale[2 * (layer * n + w) + 1] = 1.0 / (K * K);
+      gscale[2 * (layer * n + w) + 1] = phi_scale;
       group *= factor(w);
     }
   }
@@ -323,52 +327,56 @@ __global__ void __launch_bounds__(kEnergyTileThreads) energy_tile_kernel(const d
 // ------------------------------------------------------------------------
 
 
-__global__ void finalize_kernel(const FinalizeParams F) {
-  __shared__ double red[32];
-  const int t = threadIdx.x;
-  if (F.pipeline_err != nullptr && *F.pipeline_err != 0) {
-    // a backward pass did not complete: no result is better than a wrong one
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    if (t == 0) *F.energy_out = nan;
-    if (F.grad_out != nullptr)
-      for (int k = t; k < 2 * F.L * F.n; k += blockDim.x) F.grad_out[k] = nan;
+// Block 0 adds the energy; in the others a warp takes one parameter pair of a
+// wire and adds its records, lane by lane in CTA order and then over the lanes.
+// (One block for everything, a thread a pair, took 76 us at n = 20, L = 7 and
+// 146 us at n = 25, L = 6: the records of 148 to 296 CTAs one after the other.)
+constexpr int kFinalizeThreads = 256;
+__global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(const FinalizeParams F) {
+  __shared__ double red[kFinalizeThreads / 32];
+  const int t = threadIdx.x, lane = t & 31;
+  // a backward pass that did not complete: no result is better than a wrong one
+  const bool lost = F.pipeline_err != nullptr && *F.pipeline_err != 0;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  if (blockIdx.x == 0) {
+    double e = 0.0;
+    for (int i = t; i < F.num_energy_partials; i += kFinalizeThreads) e += F.energy_partials[i];
+    e = warp_sum(e);
+    if (lane == 0) red[t >> 5] = e;
+    __syncthreads();
+    if (t == 0) {
+      double s = 0.0;
+      for (int i = 0; i < kFinalizeThreads / 32; ++i) s += red[i];
+      *F.energy_out = lost ? nan : s;
+    }
     return;
   }
-  double e = 0.0;
-  for (int i = t; i < F.num_energy_partials; i += blockDim.x) e += F.energy_partials[i];
-  e = warp_sum(e);
-  if ((t & 31) == 0) red[t >> 5] = e;
-  __syncthreads();
-  if (t == 0) {
-    double s = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
-    *F.energy_out = s;
+  const int k = static_cast<int>(blockIdx.x - 1) * (kFinalizeThreads / 32) + (t >> 5);
+  if (k >= F.L * F.n) return;
+  const int layer = k / F.n, w = k % F.n;
+  if (lost) {
+    if (lane < 2) F.grad_out[2 * k + lane] = nan;
+    return;
   }
-  if (F.grad_out == nullptr) return;
-  const int np = F.L * F.n;
-  for (int k = t; k < np; k += blockDim.x) {
-    const int layer = k / F.n;
-    const int w = k % F.n;
-    if (F.theta_pass[k] < 0) continue;  // layer 0 on the layer-0 kernel
-    {
-      const int pass = F.theta_pass[k];
-      const int slot = F.theta_slot[k];
-      const double *rec = F.pass_partials + static_cast<size_t>(pass) * F.max_grid * kPartialStride;
-      double s = 0.0;
-      for (int c = 0; c < F.pass_grid[pass]; ++c) s += rec[static_cast<size_t>(c) * kPartialStride + slot];
-      F.grad_out[2 * k] = s * F.gscale[2 * k];
-    }
-    {
-      const bool alt = layer == F.phi_alt_layer && ((F.phi_alt_wires >> w) & 1u);
-      const int pass = alt ? F.phi_alt_pass : F.phi_pass[layer];
-      const double *rec = F.pass_partials + static_cast<size_t>(pass) * F.max_grid * kPartialStride;
-      double tot = 0.0, bw = 0.0;
-      for (int c = 0; c < F.pass_grid[pass]; ++c) {
-        tot += rec[static_cast<size_t>(c) * kPartialStride + kPartialTot];
-        bw += rec[static_cast<size_t>(c) * kPartialStride + kPartialPhi + w];
-      }
-      F.grad_out[2 * k + 1] = (tot - 2.0 * bw) * (alt ? 1.0 : F.gscale[2 * k + 1]);
-    }
+  if (F.theta_pass[k] < 0) return;  // layer 0 on the layer-0 kernel, or the matrix-product layers
+  const int pass = F.theta_pass[k], slot = F.theta_slot[k];
+  const bool alt = layer == F.phi_alt_layer && ((F.phi_alt_wires >> w) & 1u);
+  const int ppass = alt ? F.phi_alt_pass : F.phi_pass[layer];
+  const double *rec = F.pass_partials + static_cast<size_t>(pass) * F.max_grid * kPartialStride;
+  const double *prec = F.pass_partials + static_cast<size_t>(ppass) * F.max_grid * kPartialStride;
+  double s = 0.0, tot = 0.0, bw = 0.0;
+  const int grid = F.pass_grid[pass], pgrid = F.pass_grid[ppass];
+  for (int c = lane; c < grid; c += 32) s += rec[static_cast<size_t>(c) * kPartialStride + slot];
+  for (int c = lane; c < pgrid; c += 32) {
+    tot += prec[static_cast<size_t>(c) * kPartialStride + kPartialTot];
+    bw += prec[static_cast<size_t>(c) * kPartialStride + kPartialPhi + w];
+  }
+  s = warp_sum(s);
+  tot = warp_sum(tot);
+  bw = warp_sum(bw);
+  if (lane == 0) {
+    F.grad_out[2 * k] = s * F.gscale[2 * k];
+    F.grad_out[2 * k + 1] = (tot - 2.0 * bw) * (alt ? 1.0 : F.gscale[2 * k + 1]);
   }
 }
 
@@ -512,7 +520,8 @@ cudaError_t launch_defer_phase(const DeferPhaseArgs &A, double2 *out, cudaStream
 }
 
 cudaError_t launch_finalize(const FinalizeParams &F, cudaStream_t s) {
-  finalize_kernel<<<1, 256, 0, s>>>(F);
+  const int pairs = F.grad_out != nullptr ? F.L * F.n : 0, warps = kFinalizeThreads / 32;
+  finalize_kernel<<<1 + (pairs + warps - 1) / warps, kFinalizeThreads, 0, s>>>(F);
   return cudaGetLastError();
 }
 

@@ -176,7 +176,9 @@ __global__ void mps_tables_kernel(const MpsParams Q) {
   const int nlo = 1 << Q.m1, nhi = 1 << Q.m2;
   if (e < 1024) {
     const int k = e >> 8, v = e & 255;
-    store_mat<D>(Q.btab + e * D * D, site_chain<D>(Q.tsite, 8 * k, 8, static_cast<unsigned>(v)));
+    // (wires from n on are identities and left out)
+    const int wires = Q.n - 8 * k < 0 ? 0 : (Q.n - 8 * k < 8 ? Q.n - 8 * k : 8);
+    store_mat<D>(Q.btab + e * D * D, site_chain<D>(Q.tsite, 8 * k, wires, static_cast<unsigned>(v)));
   } else if (e < 1024 + nlo) {
     const int lo = e - 1024;
     store_mat<D>(Q.coslo + lo * D * D, site_chain<D>(Q.tsite, 12, Q.m1, static_cast<unsigned>(lo)));
@@ -190,7 +192,7 @@ __global__ void mps_tables_kernel(const MpsParams Q) {
   } else if (e < 1024 + nlo + nhi + 128 + (1 << (Q.n > 16 ? Q.n - 16 : 0))) {
     // W(x) = B2[x & 255] B3[x >> 8]: the product over wires 16..31
     const int x = e - 1024 - nlo - nhi - 128;
-    store_mat<D>(Q.wtab + x * D * D, site_chain<D>(Q.tsite, 16, 16, static_cast<unsigned>(x)));
+    store_mat<D>(Q.wtab + x * D * D, site_chain<D>(Q.tsite, 16, Q.n > 16 ? Q.n - 16 : 0, static_cast<unsigned>(x)));
   }
 }
 
@@ -774,6 +776,24 @@ __global__ void __launch_bounds__(mg4::kThreads, 1) mps_grad4_kernel(const MpsPa
   }
 }
 
+// Sum over the 64 rows of red, element t % E for every thread (64 threads): the
+// 64 / E groups of threads add their rows in order, the groups' sums are then
+// added in order.  (A tree over rows left all elements of a row to one thread.)
+template <int E>
+__device__ __forceinline__ double2 rows_sum(double2 (*red)[E], int t) {
+  constexpr int kGroups = 64 / E, kRows = 64 / kGroups;
+  const int e = t % E, g = t / E;
+  double2 s = red[g * kRows][e];
+  for (int r = 1; r < kRows; ++r) s = cadd(s, red[g * kRows + r][e]);
+  __syncthreads();
+  red[g][e] = s;
+  __syncthreads();
+  s = red[0][e];
+#pragma unroll
+  for (int k = 1; k < kGroups; ++k) s = cadd(s, red[k][e]);
+  return s;
+}
+
 // Y(lo) = sum_hi CosHi(hi) Z(lo, hi)   (blocks 0 .. 2^m1 - 1)
 // Y'(hi) = sum_lo Z(lo, hi) CosLo(lo)  (blocks 2^m1 .. 2^m1 + 2^m2 - 1)
 template <int D>
@@ -803,23 +823,25 @@ __global__ void __launch_bounds__(64) mps_coset_kernel(const MpsParams Q) {
 #pragma unroll
   for (int e = 0; e < E; ++e) red[t][e] = acc.m[e];
   __syncthreads();
-  for (int s = 32; s > 0; s >>= 1) {
-    if (t < s)
-#pragma unroll
-      for (int e = 0; e < E; ++e) red[t][e] = cadd(red[t][e], red[t + s][e]);
-    __syncthreads();
-  }
-  if (t < E) (b < nlo ? Q.ylo + b * E : Q.yhi + (b - nlo) * E)[t] = red[0][t];
+  const double2 sum = rows_sum<E>(red, t);
+  if (t < E) (b < nlo ? Q.ylo + b * E : Q.yhi + (b - nlo) * E)[t] = sum;
 }
 
-// G and F summed over the gradient kernel's CTAs, in CTA order
+// G and F summed over the gradient kernel's CTAs: a block takes 32 elements, its
+// eight warps every eighth CTA in order, then the warps' sums in order (one
+// thread an element and all CTAs took 23 us for 148 of them).
 template <int D>
-__global__ void mps_reduce_kernel(const MpsParams Q, int grid) {
+__global__ void __launch_bounds__(256) mps_reduce_kernel(const MpsParams Q, int grid) {
   constexpr int E = D * D;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * 64 * E) return;
+  __shared__ double2 part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = static_cast<int>(blockIdx.x) * 32 + lane;
   double2 s = make_double2(0.0, 0.0);
-  for (int c = 0; c < grid; ++c) s = cadd(s, Q.partials[static_cast<size_t>(c) * 2 * 64 * E + i]);
+  for (int c = warp; c < grid; c += 8) s = cadd(s, Q.partials[static_cast<size_t>(c) * 2 * 64 * E + i]);
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) s = cadd(s, part[k][lane]);
   Q.gf[i] = s;
 }
 
@@ -865,12 +887,8 @@ __global__ void __launch_bounds__(64) mps_finalize_kernel(const MpsParams Q, dou
 #pragma unroll
     for (int e = 0; e < E; ++e) red[t][b * E + e] = acc[b].m[e];
   __syncthreads();
-  for (int s = 32; s > 0; s >>= 1) {
-    if (t < s)
-      for (int e = 0; e < 2 * E; ++e) red[t][e] = cadd(red[t][e], red[t + s][e]);
-    __syncthreads();
-  }
-  if (t < 2 * E) env[t] = red[0][t];
+  const double2 sum = rows_sum<2 * E>(red, t);
+  if (t < 2 * E) env[t] = sum;
   __syncthreads();
   if (t < 2 * K) {
     const int layer = t >> 1, kind = 1 + (t & 1);
@@ -902,7 +920,7 @@ cudaError_t launch_grad_d(const MpsParams &Q, const double2 *lam, int gather, in
   mps_coset_kernel<D><<<(1 << Q.m1) + (1 << Q.m2), 64, 0, s>>>(Q);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  mps_reduce_kernel<D><<<(2 * 64 * D * D + 255) / 256, 256, 0, s>>>(Q, grid);
+  mps_reduce_kernel<D><<<2 * 64 * D * D / 32, 256, 0, s>>>(Q, grid);
   return cudaGetLastError();
 }
 
