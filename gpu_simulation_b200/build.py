@@ -66,7 +66,9 @@ def build(verbose: bool = False, ptxas_verbose: bool = False) -> Path:
         obj = BUILD / (Path(src).stem + ".o")
         objs.append(obj)
         if _newer(obj, [CSRC / src, *headers]) or ptxas_verbose:
-            cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+            # -split-compile: the many instantiations of a cluster kernel in parallel
+            split = ["-split-compile=0"] if src == "rsv_cluster.cu" else []
+            cmd = [NVCC, *ARCH, "-O3", "-lineinfo", *split, "-std=c++17", "-Xcompiler", "-fPIC",
                    "-c", str(CSRC / src), "-o", str(obj)]
             if ptxas_verbose:
                 cmd.insert(1, "-Xptxas=-v")

@@ -901,7 +901,7 @@ struct rsv_backend {
   // (rsv_ring.cu; its kept components lie in the state buffers) or the
   // cluster-resident state (rsv_cluster.cu); and the field of the last forward
   rsv::Path path = rsv::Path::kPasses;
-  rsv::ClusterShape cluster_shape{0, 4};
+  rsv::ClusterShape cluster_shape{0, 4, true};
   double forward_field = 0.0;
   rsv::DevBuf<int> tables;  // pass_grid | theta_pass | theta_slot | phi_pass
   rsv::DevBuf<int> order;   // undo order of the wires within a backward layer
@@ -1275,8 +1275,8 @@ RingParams ring_params(rsv_backend *B, const double *d_params, double *energy_ou
 ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_out, double *grad_out) {
   ClusterArgs A{};
   A.n = B->n;
-  A.log_ctas = B->cluster_shape.log_ctas;
-  A.register_bits = B->cluster_shape.register_bits;
+  A.shape = B->cluster_shape;
+  A.checkpoints = B->states.p;
   A.count = 1;
   A.item.L = A.max_layers = B->L;
   A.item.h = B->forward_field;
@@ -1286,6 +1286,13 @@ ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_
   A.grad_out = grad_out;
   return A;
 }
+
+// The cluster path's H psi of a split call, behind its checkpoints, and psi.
+double2 *cluster_lambda(rsv_backend *B) {
+  return B->states.p + cluster_checkpoint_values(B->n, B->cluster_shape, B->L);
+}
+
+double2 *cluster_psi(rsv_backend *B) { return cluster_lambda(B) + B->state_len; }
 
 // A call on the ring or the cluster path.  d_params: the angles, or null when
 // B->coef holds their cosines and sines.  keep: what a later gradient needs
@@ -1301,8 +1308,8 @@ void run_direct(rsv_backend *B, const double *d_params, bool grad, bool keep, do
   }
   ClusterArgs A = cluster_args(B, d_params, energy_out, grad ? grad_out : nullptr);
   if (keep) {
-    A.psi = state_buf(B, 0);
-    A.lam = state_buf(B, 1);
+    A.psi = cluster_psi(B);
+    A.lam = cluster_lambda(B);
     A.coef_out = d_params ? B->coef.p : nullptr;
   }
   timed(B, st, 1, 0.0, [&] { check(launch_cluster(A, st), "cluster launch"); });
@@ -1319,8 +1326,8 @@ void run_direct_backward(rsv_backend *B, double *grad_out, cudaStream_t st) {
     return;
   }
   ClusterArgs A = cluster_args(B, nullptr, nullptr, grad_out);
-  A.psi = state_buf(B, 0);
-  A.lam = state_buf(B, 1);
+  A.psi = cluster_psi(B);
+  A.lam = cluster_lambda(B);
   A.resume = 1;
   timed(B, st, 3, 0.0, [&] { check(launch_cluster(A, st), "cluster launch"); });
 }
@@ -1534,10 +1541,14 @@ struct rsv_batch {
   // that gave slots, or set them or a cluster size, chose the persistent kernel.
   bool resident = true;
   struct Class {
-    int n, first, count, max_layers;
+    int n, first, count, max_layers, clusters;
+    rsv::ClusterShape shape;
+    size_t checkpoint;  // first value of the class's checkpoints
   };
   std::vector<Class> classes;
-  unsigned int fits = 0;  // qubit counts whose clusters fit the device
+  int fits[rsv::kBatchMaxQubits + 1] = {};  // clusters the device holds, per qubit count
+  rsv::DevBuf<double2> d_checkpoints;
+  rsv::DevBuf<int> d_counters;  // per class: circuits taken
   rsv::DevBuf<rsv::ClusterItem> d_items;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> joined;
@@ -1625,12 +1636,18 @@ void batch_group(rsv_batch *Bt) {
 // How a batch spreads its circuits, for throughput: 16 amplitudes a thread from
 // 10 qubits on, as few CTAs as hold the state (4096 amplitudes each).  At L = 8
 // and as many CTAs as an SM holds: n = 9 5 us a circuit and SM (16 a thread 5.9),
-// n = 10 10.8 (8 a thread 15.5), n = 11 25 (49), n = 12 90.
+// n = 10 10.8 (8 a thread 15.5), n = 11 25 (49), n = 12 90.  With checkpoints where
+// un-computing psi means moving it between CTAs: 600 circuits of n = 13, L = 12
+// 2.44 ms against 2.60, 150 of n = 15 3.83 against 4.35, 80 of n = 16 4.81 against 5.05.
 ClusterShape batch_shape_for(int n) {
-  if (n <= 8) return {0, 2};
-  if (n == 9) return {0, 3};
-  return {std::max(0, n - kTileBits), 4};
+  if (n <= 8) return {0, 2, false};
+  if (n == 9) return {0, 3, false};
+  return {std::max(0, n - kTileBits), 4, n > kTileBits};
 }
+
+// Checkpoints of all classes together (16 layers of all qubit counts from 13 on,
+// 148 SMs: 2.5 GB); a class beyond that un-computes psi.
+constexpr size_t kBatchCheckpointBytes = size_t{4} << 30;
 
 // The circuits by qubit count (largest first) and depth (deepest first); false
 // where the device does not hold a cluster of some class.
@@ -1646,13 +1663,15 @@ bool batch_classes(rsv_batch *Bt, const std::vector<BatchCircuit> &circ) {
   for (int c : order) {
     const BatchCircuit &C = circ[static_cast<size_t>(c)];
     if (Bt->classes.empty() || Bt->classes.back().n != C.n) {
-      if (!((Bt->fits >> C.n) & 1)) {  // asked once a qubit count, for the deepest circuits
-        int clusters = 0;
-        check(cluster_capacity(C.n, batch_shape_for(C.n), kBatchMaxLayers, &clusters), "cluster capacity");
-        if (clusters < 1) return false;
-        Bt->fits |= 1u << C.n;
-      }
-      Bt->classes.push_back({C.n, static_cast<int>(items.size()), 0, C.L});
+      int &fit = Bt->fits[C.n];  // asked once a qubit count, for the deepest circuits
+      if (fit == 0) check(cluster_capacity(C.n, batch_shape_for(C.n), kBatchMaxLayers, &fit), "cluster capacity");
+      if (fit < 1) return false;
+      rsv_batch::Class k{};
+      k.n = C.n;
+      k.first = static_cast<int>(items.size());
+      k.max_layers = C.L;
+      k.shape = batch_shape_for(C.n);
+      Bt->classes.push_back(k);
     }
     ++Bt->classes.back().count;
     ClusterItem it{};
@@ -1662,6 +1681,24 @@ bool batch_classes(rsv_batch *Bt, const std::vector<BatchCircuit> &circ) {
     it.h = C.h;
     items.push_back(it);
   }
+  // checkpoints for as many clusters of each class as the device holds
+  size_t values = 0;
+  for (auto &k : Bt->classes) {
+    k.clusters = std::min(k.count, Bt->fits[k.n]);
+    const size_t v = cluster_checkpoint_values(k.n, k.shape, k.max_layers) * static_cast<size_t>(k.clusters);
+    if ((values + v) * sizeof(double2) > kBatchCheckpointBytes) k.shape.checkpoints = false;
+    if (!k.shape.checkpoints) continue;
+    k.checkpoint = values;
+    values += v;
+  }
+  try {
+    if (Bt->d_checkpoints.count < values) Bt->d_checkpoints.alloc(values);
+  } catch (const Error &e) {
+    if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
+    cudaGetLastError();  // clear the allocation failure; psi is un-computed
+    for (auto &k : Bt->classes) k.shape.checkpoints = false;
+  }
+  if (Bt->d_counters.p == nullptr) Bt->d_counters.alloc(kBatchMaxQubits + 1);
   while (Bt->side.size() + 1 < Bt->classes.size()) {
     // the larger circuits' clusters go first where both wait for SMs
     int least = 0, greatest = 0;
@@ -1731,11 +1768,14 @@ void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *
   if (Bt->resident) {
     auto launch = [&](const rsv_batch::Class &c, cudaStream_t s) {
       ClusterArgs A{};
-      const ClusterShape h = batch_shape_for(c.n);
       A.n = c.n;
-      A.log_ctas = h.log_ctas;
-      A.register_bits = h.register_bits;
+      A.shape = c.shape;
       A.count = c.count;
+      if (c.shape.checkpoints) {
+        A.clusters = c.clusters;
+        A.counter = Bt->d_counters.p + c.n;
+        A.checkpoints = Bt->d_checkpoints.p + c.checkpoint;
+      }
       A.items = Bt->d_items.p + c.first;
       A.max_layers = c.max_layers;
       A.params = d_params;
@@ -1743,6 +1783,7 @@ void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *
       A.grad_out = d_grad;
       check(launch_cluster(A, s), "batch launch");
     };
+    check(cudaMemsetAsync(Bt->d_counters.p, 0, (kBatchMaxQubits + 1) * sizeof(int), st), "batch counter reset");
     const size_t others = Bt->classes.size() - 1;
     if (others > 0) check(cudaEventRecord(Bt->forked, st), "cudaEventRecord");
     launch(Bt->classes[0], st);
@@ -1996,12 +2037,14 @@ bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 16 && L == 5)
 // CTA (n = 9 23.6 us, 8 a thread 24.8, 16 a thread 47), 10 and 11 qubits 8 a
 // thread (31 and 51 us; 4 a thread 35 and 55), 12 and 13 on 8 CTAs (64 and 86
 // us; on one or two 90 and 180), then 16 CTAs (14 qubits 120 us against 137 on
-// 8, 16 qubits 293 against 336 on the tile passes).
+// 8).  Checkpoints pay from 15 qubits on, where un-computing psi means moving it
+// between CTAs (15 qubits 163 us against 170, 16 qubits 258 against 293; 14
+// qubits 123 against 120, 12 qubits 72 against 64).
 ClusterShape cluster_shape_for(int n) {
-  if (n <= 9) return {0, 2};
-  if (n <= 11) return {0, 3};
-  if (n <= 13) return {3, 3};
-  return {4, 4};
+  if (n <= 9) return {0, 2, false};
+  if (n <= 11) return {0, 3, false};
+  if (n <= 13) return {3, 3, false};
+  return {4, 4, n >= 15};
 }
 
 // What runs a backend's calls.  A caller that chose a backward schedule, fewer
@@ -2057,11 +2100,14 @@ void setup_plan(rsv_backend *B, int mode) {
   Plan pl = make_plan(B->n, B->L, B->sms, want, B->analytic_layers, B->force_c);
   B->state_len = size_t{1} << pl.phys;
   B->path = choose_path(B, mode);
-  const size_t ring_values =
-      B->path == Path::kRing ? 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs : 0;
-  if (ring_values > static_cast<size_t>(pl.num_bufs) * B->state_len) {
+  size_t values = 0;
+  if (B->path == Path::kRing)
+    values = 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs;
+  else if (B->path == Path::kCluster)
+    values = cluster_checkpoint_values(B->n, B->cluster_shape, B->L) + 2 * B->state_len;
+  if (values > static_cast<size_t>(pl.num_bufs) * B->state_len) {
     try {
-      B->states.alloc(ring_values);
+      B->states.alloc(values);
     } catch (const Error &e) {
       if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
       cudaGetLastError();  // clear the allocation failure
@@ -2076,7 +2122,7 @@ void setup_plan(rsv_backend *B, int mode) {
     pl = make_plan(B->n, B->L, B->sms, false, B->analytic_layers, B->force_c);
     B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
   }
-  // (zero padding for n < 12; the ring's components need none)
+  // (zero padding for n < 12; the other paths need none)
   check(cudaMemset(B->states.p, 0, std::min(B->states.count, static_cast<size_t>(pl.num_bufs) * B->state_len) *
                                        sizeof(double2)),
         "state memset");

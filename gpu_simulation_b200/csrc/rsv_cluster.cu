@@ -34,6 +34,13 @@
 // them is undone.  phi sums are taken on the true vectors at the layer's start:
 // sum_i z_w(i) Im(conj(lambda_i) psi_i).
 //
+// With checkpoints (CK) the forward writes psi behind every layout's rotations
+// to memory, 2^R amplitudes a thread in the thread's own order, and the backward
+// reads them back instead of un-computing psi: only lambda is rotated and
+// exchanged, and a theta or phi sum with a checkpoint needs no correction (psi
+// there is 1 / K_S of what un-computing gives, which is what the sum lacks).
+// Layer 0's psi is the product state and is un-computed.
+//
 // Sums go through fixed orders (lanes, warps, CTAs): equal inputs give equal bits.
 //
 // Bound by latency up to 12 qubits (one launch against one a layer and pass:
@@ -261,13 +268,17 @@ __device__ __forceinline__ double warp_sums32(double (&v)[32], int lane) {
   return v[0];
 }
 
-template <int n_, int R_, int C_>
-__global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(const __grid_constant__ ClusterArgs A) {
-  using G = Geo<n_, R_, C_>;
+template <bool V>
+struct Flag {
+  static constexpr bool value = V;
+};
+
+// One circuit on this cluster; `ck`: this CTA's checkpoints.
+template <typename G, bool CK>
+__device__ __forceinline__ void run_circuit(const ClusterArgs &A, const ClusterItem item, unsigned char *smem,
+                                            double2 *ck) {
   constexpr int n = G::n, N = G::N, R = G::R, C = G::C, m = G::m, K = G::K, NR = G::NR, nt = G::tables;
   constexpr int threads = G::threads, warps = G::warps;
-  extern __shared__ __align__(128) unsigned char smem[];
-  const ClusterItem item = A.items ? A.items[blockIdx.x >> C] : A.item;
   const int L = item.L;
   const unsigned rank = blockIdx.x & ((1u << C) - 1), tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -384,6 +395,19 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
   const unsigned top_turn = C > 0 ? rank : 0u;
 
   double2 psi[NR], lam[NR];
+  // a thread's amplitudes behind layout k of layer l (l >= 1)
+  auto checkpoint = [&](int l, int k) { return ck + (static_cast<size_t>(l) * K + k) * (NR * threads) + tid; };
+  auto save = [&](int l, int k) {
+    double2 *p = checkpoint(l, k);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) p[r * threads] = psi[r];
+  };
+  auto restore = [&](int l, int k) {
+    const double2 *p = checkpoint(l, k);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) psi[r] = p[r * threads];
+  };
+  const bool keep = A.grad_out != nullptr || A.lam != nullptr;
   if (!A.resume) {
     // ---- layer 0: the product state, in layout K-1
     {
@@ -405,6 +429,7 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
 #pragma unroll
         for (int j = 0; j < R; ++j)
           if (G::wire(k, j) >= 0) rotate<R>(psi, j, factor(rot, k, j));
+        if (CK && keep) save(l, k);
         if (k == K - 1) break;
         if (k + 1 < K - 1) {
           store_own<G>(psi, bufP, k, own[k] ^ swaps(flip, k, [&](int j) { return G::own_bit(k, j); }));
@@ -490,10 +515,10 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
     }
     energy = warp_sum(energy);
     if (lane == 0) T.red[warp] = energy;
-    if (A.psi) {
+    if (A.lam) {
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
-        A.psi[x0 ^ static_cast<unsigned>(r)] = psi[r];
+        if (!CK) A.psi[x0 ^ static_cast<unsigned>(r)] = psi[r];
         A.lam[x0 ^ static_cast<unsigned>(r)] = lam[r];
       }
     }
@@ -512,7 +537,7 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
   } else {
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-      psi[r] = A.psi[x0 ^ static_cast<unsigned>(r)];
+      if (!CK) psi[r] = A.psi[x0 ^ static_cast<unsigned>(r)];
       lam[r] = A.lam[x0 ^ static_cast<unsigned>(r)];
     }
   }
@@ -532,29 +557,39 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
   };
 
   // ---- backward (the slots are free at the start of every layer)
-#pragma unroll 1
-  for (int l = L - 1; l >= 0; --l) {
-    push<G>(psi, smP, unring, unring_bit);
-    push<G>(lam, smL, unring, unring_bit);
-    sync_all<G>();
-    if (l < L - 1) gather(l + 1);
+  auto undo_layer = [&](int l, auto mode) {
+    constexpr bool uncompute = decltype(mode)::value;
     const unsigned flip = T.flip[l];
     const unsigned swap = swaps(flip, K - 1, [](int j) { return G::own_bit(K - 1, j); });
-    load_own<G>(psi, bufP, K - 1, own[K - 1] ^ swap);
+    if (!CK) push<G>(psi, smP, unring, unring_bit);
+    push<G>(lam, smL, unring, unring_bit);
+    if constexpr (!uncompute) {
+      restore(l, K - 1);
+    } else if constexpr (CK) {
+      {  // the product state; registers are numbered before J's swap
+        const double2 z = phase_base(T.prod);
+        const unsigned turn = top_turn ^ ((flip >> (N - R)) & (NR - 1));
+#pragma unroll
+        for (int r = 0; r < NR; ++r) psi[r] = cmul(z, T.prod[16 * (nt - 1) + (r ^ turn)]);
+      }
+    }
+    sync_all<G>();
+    if (l < L - 1) gather(l + 1);
+    if (!CK) load_own<G>(psi, bufP, K - 1, own[K - 1] ^ swap);
     load_own<G>(lam, bufL, K - 1, own[K - 1] ^ swap);
     arrive<G>();
-    // phi sums: per register bit and in total
+    // D^+ K on lambda, and on a psi that is un-computed; phi sums on the true
+    // vectors, or on lambda behind D^+ K and the checkpoint before D
     double tot = 0.0, one[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) one[j] = 0.0;
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
+    auto phi_sum = [&](int r) {
       const double q = fma(lam[r].x, psi[r].y, -lam[r].y * psi[r].x);
       tot += q;
 #pragma unroll
       for (int j = 0; j < R; ++j)
         if ((r >> j) & 1) one[j] += q;
-    }
+    };
     {
       const double2 *tab = T.phase + static_cast<size_t>(l) * nt * 16;
       double2 z = phase_base(tab);
@@ -563,8 +598,12 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const double2 f = cmul(z, tab[16 * (nt - 1) + (r ^ top_turn)]);
-        psi[r] = cmul_conj(psi[r], f);
+        if constexpr (uncompute) {
+          phi_sum(r);
+          psi[r] = cmul_conj(psi[r], f);
+        }
         lam[r] = cmul_conj(lam[r], f);
+        if constexpr (!uncompute) phi_sum(r);
       }
     }
     double sums[32];
@@ -579,28 +618,29 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
           const double s = theta_sum<R>(psi, lam, j);
           sums[G::wire(k, j) & 15] = turned(k, j) ? -s : s;
         }
+      if (!uncompute && k > 0) restore(l, k - 1);  // in flight during lambda's exchange
       if (k > 0 || l > 0) {
 #pragma unroll
         for (int j = 0; j < R; ++j)
           if (G::wire(k, j) >= 0) {
             const double f = -factor(rot, k, j);
-            rotate<R>(psi, j, f);
+            if (uncompute) rotate<R>(psi, j, f);
             rotate<R>(lam, j, f);
           }
       }
       if (k == 0) break;
       if (k == K - 1) {
         wait<G>();
-        push<G>(psi, smP, down, down_bit);
+        if (uncompute) push<G>(psi, smP, down, down_bit);
         push<G>(lam, smL, down, down_bit);
         sync_all<G>();
       } else {
-        store_own<G>(psi, bufP, k, own[k]);
+        if (uncompute) store_own<G>(psi, bufP, k, own[k]);
         store_own<G>(lam, bufL, k, own[k]);
         sync_cta<G>();
       }
       const unsigned next = own[k - 1] ^ swaps(flip, k - 1, [&](int j) { return G::own_bit(k - 1, j); });
-      load_own<G>(psi, bufP, k - 1, next);
+      if (uncompute) load_own<G>(psi, bufP, k - 1, next);
       load_own<G>(lam, bufL, k - 1, next);
     }
     arrive<G>();
@@ -614,6 +654,14 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
     else T.red[(l & 1) * 32 * warps + 32 * warp + lane] = s;  // (read while the next layer fills the other half)
     if (lane == kRecTotal) T.tot[l * warps + warp] = s;
     wait<G>();  // every slot is read
+  };
+  if constexpr (CK) {
+#pragma unroll 1
+    for (int l = L - 1; l > 0; --l) undo_layer(l, Flag<false>{});
+    undo_layer(0, Flag<true>{});
+  } else {
+#pragma unroll 1
+    for (int l = L - 1; l >= 0; --l) undo_layer(l, Flag<true>{});
   }
   sync_all<G>();
   gather(0);
@@ -631,7 +679,7 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
       double s[2] = {1.0, 1.0};  // prod (1 + k^2) over the wires still pending there
       const int pending = G::pending(w);
       for (int v = 0; v < pending && v < n; ++v) s[v & 1] *= fma(T.rot[l * N + v], T.rot[l * N + v], 1.0);
-      out *= s[0] * s[1];
+      if (!CK || l == 0) out *= s[0] * s[1];
     } else {
       // sum of z_w: the total less twice the sum over the amplitudes with bit w
       double tot = 0.0, b = 0.0;
@@ -662,10 +710,48 @@ __global__ void __launch_bounds__(Geo<n_, R_, C_>::threads, 1) cluster_kernel(co
   sync_all<G>();  // records stay until they are read
 }
 
-template <int n, int R, int C>
+__device__ __forceinline__ void store_cluster_u32(unsigned addr, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+template <int n, int R, int C, bool CK>
+__global__ void __launch_bounds__(Geo<n, R, C>::threads, 1) cluster_kernel(const __grid_constant__ ClusterArgs A) {
+  using G = Geo<n, R, C>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const unsigned cluster = blockIdx.x >> C, rank = blockIdx.x & ((1u << C) - 1);
+  double2 *ck = CK ? A.checkpoints + (static_cast<size_t>(cluster) * G::ctas + rank) * A.max_layers *
+                                         (static_cast<size_t>(G::K) * G::NR * G::threads)
+                   : nullptr;
+  unsigned size;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(size));
+  int *next = reinterpret_cast<int *>(smem + size - 16);
+  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(next));
+  for (;;) {
+    int i = static_cast<int>(cluster);
+    if (A.counter != nullptr) {  // as many clusters as fit take the circuits in order
+      if (rank == 0 && threadIdx.x == 0) {
+        i = atomicAdd(A.counter, 1);
+        for (int k = 0; k < G::ctas; ++k) store_cluster_u32(C > 0 ? cluster_address(at, k) : at, i);
+      }
+      sync_all<G>();
+      i = *reinterpret_cast<volatile int *>(next);
+      if (i >= A.count) return;
+    }
+    run_circuit<G, CK>(A, A.items ? A.items[i] : A.item, smem, ck);
+    if (A.counter == nullptr) return;
+    sync_all<G>();  // (an energy-only circuit's last reads; everyone has read `next`)
+  }
+}
+
+template <int n, int R, int C, bool CK>
 struct Shape {
   using G = Geo<n, R, C>;
-  static bool is(int qubits, ClusterShape h) { return qubits == n && h.register_bits == R && h.log_ctas == C; }
+  static bool is(int qubits, ClusterShape h) {
+    return qubits == n && h.register_bits == R && h.log_ctas == C && h.checkpoints == CK;
+  }
+  static size_t checkpoint_values(int max_layers) {
+    return CK ? (static_cast<size_t>(max_layers) * G::K) << G::N : 0;
+  }
   static size_t smem(int max_layers) {
     const size_t bufs = size_t{32} << G::m;
     size_t most = 0;  // (a circuit of fewer layers may be the one whose pairs need room of their own)
@@ -673,11 +759,11 @@ struct Shape {
       const size_t b = bufs + table_bytes<G>(L) + (trig_bytes(n, L) <= bufs ? 0 : trig_bytes(n, L));
       if (b > most) most = b;
     }
-    return most;
+    return most + 16;  // (the next circuit's number)
   }
-  static void fill(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int max_layers, int count) {
+  static void fill(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int max_layers, int clusters) {
     cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3(static_cast<unsigned>(count) << C);
+    cfg.gridDim = dim3(static_cast<unsigned>(clusters) << C);
     cfg.blockDim = dim3(static_cast<unsigned>(G::threads));
     cfg.dynamicSmemBytes = smem(max_layers);
     at.id = cudaLaunchAttributeClusterDimension;
@@ -689,13 +775,13 @@ struct Shape {
   // both attributes belong to the device: set once on each
   static cudaError_t configure() {
     static std::atomic<unsigned long long> smem_done{0}, size_done{0};
-    cudaError_t e = set_smem_limit_once(cluster_kernel<n, R, C>, kMostSmem, smem_done);
+    cudaError_t e = set_smem_limit_once(cluster_kernel<n, R, C, CK>, kMostSmem, smem_done);
     if (e != cudaSuccess || C < 4) return e;
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     const unsigned long long bit = dev < 64 ? (1ull << dev) : 0ull;
     if (bit != 0 && (size_done.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
-    e = cudaFuncSetAttribute(cluster_kernel<n, R, C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(cluster_kernel<n, R, C, CK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess && bit != 0) size_done.fetch_or(bit, std::memory_order_acq_rel);
     return e;
   }
@@ -704,9 +790,9 @@ struct Shape {
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
-    fill(cfg, at, A.max_layers, A.count);
+    fill(cfg, at, A.max_layers, A.counter ? A.clusters : A.count);
     cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, cluster_kernel<n, R, C>, A);
+    return cudaLaunchKernelEx(&cfg, cluster_kernel<n, R, C, CK>, A);
   }
   static cudaError_t capacity(int max_layers, int *clusters) {
     if (smem(max_layers) > kMostSmem) return cudaSuccess;
@@ -715,7 +801,7 @@ struct Shape {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     fill(cfg, at, max_layers, 1);
-    return cudaOccupancyMaxActiveClusters(clusters, cluster_kernel<n, R, C>, &cfg);
+    return cudaOccupancyMaxActiveClusters(clusters, cluster_kernel<n, R, C, CK>, &cfg);
   }
 };
 
@@ -729,28 +815,32 @@ bool with_shape(int n, ClusterShape h, F &&f) {
       f(shape);
     }
   };
-  one(Shape<2, 2, 0>{});
-  one(Shape<3, 2, 0>{});
-  one(Shape<4, 2, 0>{});
-  one(Shape<5, 2, 0>{});
-  one(Shape<6, 2, 0>{});
-  one(Shape<7, 2, 0>{});
-  one(Shape<8, 2, 0>{});
-  one(Shape<9, 2, 0>{});
-  one(Shape<9, 3, 0>{});
-  one(Shape<10, 3, 0>{});
-  one(Shape<10, 4, 0>{});
-  one(Shape<11, 3, 0>{});
-  one(Shape<11, 4, 0>{});
-  one(Shape<12, 3, 3>{});
-  one(Shape<12, 4, 0>{});
-  one(Shape<13, 3, 3>{});
-  one(Shape<13, 4, 1>{});
-  one(Shape<14, 4, 4>{});
-  one(Shape<14, 4, 2>{});
-  one(Shape<15, 4, 4>{});
-  one(Shape<15, 4, 3>{});
-  one(Shape<16, 4, 4>{});
+  one(Shape<2, 2, 0, false>{});
+  one(Shape<3, 2, 0, false>{});
+  one(Shape<4, 2, 0, false>{});
+  one(Shape<5, 2, 0, false>{});
+  one(Shape<6, 2, 0, false>{});
+  one(Shape<7, 2, 0, false>{});
+  one(Shape<8, 2, 0, false>{});
+  one(Shape<9, 2, 0, false>{});
+  one(Shape<9, 3, 0, false>{});
+  one(Shape<10, 3, 0, false>{});
+  one(Shape<10, 4, 0, false>{});
+  one(Shape<11, 3, 0, false>{});
+  one(Shape<11, 4, 0, false>{});
+  one(Shape<12, 3, 3, false>{});
+  one(Shape<12, 4, 0, false>{});
+  one(Shape<13, 3, 3, false>{});
+  one(Shape<13, 4, 1, false>{});
+  one(Shape<13, 4, 1, true>{});
+  one(Shape<14, 4, 4, false>{});
+  one(Shape<14, 4, 2, false>{});
+  one(Shape<14, 4, 2, true>{});
+  one(Shape<15, 4, 4, true>{});
+  one(Shape<15, 4, 3, false>{});
+  one(Shape<15, 4, 3, true>{});
+  one(Shape<16, 4, 4, false>{});
+  one(Shape<16, 4, 4, true>{});
   return found;
 }
 
@@ -763,7 +853,7 @@ bool cluster_shape_built(int n, ClusterShape h) {
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s) {
   if (A.count < 1) return cudaSuccess;
   cudaError_t e = cudaErrorInvalidValue;
-  with_shape(A.n, ClusterShape{A.log_ctas, A.register_bits}, [&](auto shape) { e = decltype(shape)::launch(A, s); });
+  with_shape(A.n, A.shape, [&](auto shape) { e = decltype(shape)::launch(A, s); });
   return e;
 }
 
@@ -772,6 +862,12 @@ cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *cluster
   cudaError_t e = cudaSuccess;
   with_shape(n, h, [&](auto shape) { e = decltype(shape)::capacity(max_layers, clusters); });
   return e;
+}
+
+size_t cluster_checkpoint_values(int n, ClusterShape h, int max_layers) {
+  size_t v = 0;
+  with_shape(n, h, [&](auto shape) { v = decltype(shape)::checkpoint_values(max_layers); });
+  return v;
 }
 
 }  // namespace rsv

@@ -18,11 +18,20 @@ struct ClusterItem {
   double h;
 };
 
+// How a launch spreads a circuit: 2^log_ctas CTAs, 2^register_bits amplitudes a
+// thread; with checkpoints the backward reads psi from memory.
+struct ClusterShape {
+  int log_ctas, register_bits;
+  bool checkpoints;
+};
+
 struct ClusterArgs {
   int n;
-  int log_ctas;                // CTAs of a cluster (= of a circuit): 2^log_ctas
-  int register_bits;           // amplitudes of a thread: 2^register_bits
+  ClusterShape shape;
   int count;                   // circuits
+  int clusters;                // with a counter: clusters that take them in turn
+  int *counter;                // or null: one cluster a circuit
+  double2 *checkpoints;        // clusters * cluster_checkpoint_values(n, shape, max_layers)
   const ClusterItem *items;    // [count], or null: the one circuit `item`
   ClusterItem item;
   int max_layers;              // largest L of the circuits
@@ -31,17 +40,15 @@ struct ClusterArgs {
   double4 *coef_out;           // or null: the one circuit's are written here
   double *energy_out;          // or null
   double *grad_out;            // or null: no backward
-  // One circuit only: the forward call leaves psi and H psi here, and with
-  // `resume` a later call starts from them and runs the backward alone.
+  // One circuit only: the forward call leaves psi (without checkpoints) and
+  // H psi here, and with `resume` a later call starts from them (and the
+  // checkpoints) and runs the backward alone.
   double2 *psi, *lam;
   int resume;
 };
 
-// How a launch spreads a circuit: 2^log_ctas CTAs, 2^register_bits amplitudes a thread.
-struct ClusterShape {
-  int log_ctas, register_bits;
-};
 bool cluster_shape_built(int n, ClusterShape h);
+size_t cluster_checkpoint_values(int n, ClusterShape h, int max_layers);
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s);
 // Clusters of that shape that fit the device at once (0: none).
 cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *clusters);
