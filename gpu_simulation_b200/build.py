@@ -27,9 +27,9 @@ CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
-CU_SOURCES = ["rsv_kernels.cu", "rsv_pass.cu", "rsv_pass_half.cu", "rsv_layer0.cu", "rsv_mps.cu", "rsv_noalloc.cu", "rsv_pass_tma.cu", "rsv_batch.cu", "rsv_mlp.cu", "rsv_gate.cu", "rsv_dense.cu", "rsv_shard.cu", "rsv_ring.cu", "rsv_cluster.cu"]
+CU_SOURCES = ["rsv_kernels.cu", "rsv_pass.cu", "rsv_pass_half.cu", "rsv_layer0.cu", "rsv_mps.cu", "rsv_noalloc.cu", "rsv_pass_tma.cu", "rsv_batch.cu", "rsv_mlp.cu", "rsv_gate.cu", "rsv_dense.cu", "rsv_shard.cu", "rsv_ring.cu", "rsv_cluster.cu", "rsv_tiles.cu"]
 CPP_SOURCES = ["rsv_backend.cpp", "rsv_mlp_host.cpp"]
-HEADERS = ["rsv_device.cuh", "rsv_types.h", "rsv_launch.h", "rsv_workspace.h", "rsv_tma.h", "rsv_tile.cuh", "rsv_batch.h", "rsv_mlp.h", "rsv_gate.h", "rsv_dense.h", "rsv_ring.h", "rsv_cluster.h"]
+HEADERS = ["rsv_device.cuh", "rsv_types.h", "rsv_launch.h", "rsv_workspace.h", "rsv_tma.h", "rsv_tile.cuh", "rsv_batch.h", "rsv_mlp.h", "rsv_gate.h", "rsv_dense.h", "rsv_ring.h", "rsv_cluster.h", "rsv_resident.cuh"]
 
 
 def _ext_suffix() -> str:
@@ -66,8 +66,8 @@ def build(verbose: bool = False, ptxas_verbose: bool = False) -> Path:
         obj = BUILD / (Path(src).stem + ".o")
         objs.append(obj)
         if _newer(obj, [CSRC / src, *headers]) or ptxas_verbose:
-            # -split-compile: the many instantiations of a cluster kernel in parallel
-            split = ["-split-compile=0"] if src == "rsv_cluster.cu" else []
+            # -split-compile: the many instantiations of the two kernels in parallel
+            split = ["-split-compile=0"] if src in ("rsv_cluster.cu", "rsv_tiles.cu") else []
             cmd = [NVCC, *ARCH, "-O3", "-lineinfo", *split, "-std=c++17", "-Xcompiler", "-fPIC",
                    "-c", str(CSRC / src), "-o", str(obj)]
             if ptxas_verbose:

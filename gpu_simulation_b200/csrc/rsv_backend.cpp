@@ -1276,7 +1276,7 @@ ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_
   ClusterArgs A{};
   A.n = B->n;
   A.shape = B->cluster_shape;
-  A.checkpoints = B->states.p;
+  A.memory = B->states.p;
   A.count = 1;
   A.item.L = A.max_layers = B->L;
   A.item.h = B->forward_field;
@@ -1287,9 +1287,9 @@ ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_
   return A;
 }
 
-// The cluster path's H psi of a split call, behind its checkpoints, and psi.
+// The cluster path's H psi of a split call, behind the clusters' own memory, and psi.
 double2 *cluster_lambda(rsv_backend *B) {
-  return B->states.p + cluster_checkpoint_values(B->n, B->cluster_shape, B->L);
+  return B->states.p + cluster_memory_values(B->n, B->cluster_shape, B->L);
 }
 
 double2 *cluster_psi(rsv_backend *B) { return cluster_lambda(B) + B->state_len; }
@@ -1543,11 +1543,11 @@ struct rsv_batch {
   struct Class {
     int n, first, count, max_layers, clusters;
     rsv::ClusterShape shape;
-    size_t checkpoint;  // first value of the class's checkpoints
+    size_t vectors;  // first value of the class's vectors
   };
   std::vector<Class> classes;
-  int fits[rsv::kBatchMaxQubits + 1] = {};  // clusters the device holds, per qubit count
-  rsv::DevBuf<double2> d_checkpoints;
+  int fits[rsv::kBatchMaxQubits + 1][5] = {};  // clusters the device holds, per qubit count and log2 of their CTAs
+  rsv::DevBuf<double2> d_vectors;  // of the tiled classes' circuits
   rsv::DevBuf<int> d_counters;  // per class: circuits taken
   rsv::DevBuf<rsv::ClusterItem> d_items;
   std::vector<cudaStream_t> side;
@@ -1633,21 +1633,77 @@ void batch_group(rsv_batch *Bt) {
   Bt->num_groups = static_cast<int>(groups.size());
 }
 
-// How a batch spreads its circuits, for throughput: 16 amplitudes a thread from
-// 10 qubits on, as few CTAs as hold the state (4096 amplitudes each).  At L = 8
-// and as many CTAs as an SM holds: n = 9 5 us a circuit and SM (16 a thread 5.9),
-// n = 10 10.8 (8 a thread 15.5), n = 11 25 (49), n = 12 90.  With checkpoints where
-// un-computing psi means moving it between CTAs: 600 circuits of n = 13, L = 12
-// 2.44 ms against 2.60, 150 of n = 15 3.83 against 4.35, 80 of n = 16 4.81 against 5.05.
-ClusterShape batch_shape_for(int n) {
-  if (n <= 8) return {0, 2, false};
-  if (n == 9) return {0, 3, false};
-  return {std::max(0, n - kTileBits), 4, n > kTileBits};
+// The ways a batch can spread circuits of n qubits, with what a layer takes in
+// us: `latency` of a circuit that has its CTAs to itself, `work` of all SMs'
+// time on a busy device (SMs x time / circuits; L = 8, 148 SMs).  One CTA up to
+// 12 qubits, 16 amplitudes a thread from 10 on (L = 8, a circuit and SM: n = 9 5
+// us, 16 a thread 5.9; n = 10 10.8, 8 a thread 15.5; n = 11 25, 49; n = 12 90).
+// Above that tiled on 1 to 2^(n-12) CTAs: the work is that of one CTA until each
+// has one or two tiles, where waiting for one another shows.  Circuits in
+// registers on the same number of CTAs need twice the SM time and are not offered
+// (n = 16: 780 us a layer; 148 circuits 6.25 ms against 2.67); on more CTAs they
+// have the shortest latency for 13 and 14 qubits.
+struct BatchShape {
+  ClusterShape shape;
+  double latency, work;
+};
+std::vector<BatchShape> batch_shapes(int n) {
+  switch (n) {
+    case 9: return {{{0, 3, false}, 0.6, 0.6}};
+    case 10: return {{{0, 4, false}, 1.4, 1.4}};
+    case 11: return {{{0, 4, false}, 3.1, 3.1}};
+    case 12: return {{{0, 4, false}, 11, 11}};
+    case 13: return {{{0, 4, false, true}, 31, 33}, {{1, 4, false, true}, 21, 41}, {{3, 3, false}, 11, 88}};
+    case 14:
+      return {{{0, 4, false, true}, 62, 71}, {{1, 4, false, true}, 34, 73}, {{2, 4, false, true}, 21, 83},
+              {{4, 4, false}, 15, 277}};
+    case 15:
+      return {{{0, 4, false, true}, 122, 153}, {{1, 4, false, true}, 67, 147}, {{2, 4, false, true}, 36, 145},
+              {{3, 4, false, true}, 21, 190}};
+    case 16:
+      return {{{0, 4, false, true}, 250, 350}, {{1, 4, false, true}, 131, 334}, {{2, 4, false, true}, 71, 320},
+              {{3, 4, false, true}, 37, 340},  {{4, 4, false, true}, 23, 494}};
+    default: return {{{0, 2, false}, 0.3, 0.3}};
+  }
 }
 
-// Checkpoints of all classes together (16 layers of all qubit counts from 13 on,
-// 148 SMs: 2.5 GB); a class beyond that un-computes psi.
-constexpr size_t kBatchCheckpointBytes = size_t{4} << 30;
+// The shape of each class: what ends the batch soonest.  That is the work of
+// all classes spread over the SMs, or the class's own rounds of circuits (where
+// all are equally deep and rounds do not blur), or its deepest circuit, and a
+// part of the last while the device runs empty.  (148 circuits of n = 16, L = 8:
+// 2.80, 2.67, 3.11, 2.99 and 4.06 ms on 1 to 16 CTAs each, 8 circuits 1.99, 1.05,
+// 0.57, 0.30 and 0.38.)
+void batch_choose_shapes(std::vector<rsv_batch::Class> &classes, const std::vector<ClusterItem> &items, int sms) {
+  double total = 0.0;
+  std::vector<double> layers;
+  for (const auto &k : classes) {
+    double sum = 0.0;
+    for (int i = 0; i < k.count; ++i) sum += items[static_cast<size_t>(k.first + i)].L;
+    layers.push_back(sum);
+    total += batch_shapes(k.n)[0].work * sum;
+  }
+  for (size_t c = 0; c < classes.size(); ++c) {
+    auto &k = classes[c];
+    const bool even = items[static_cast<size_t>(k.first + k.count - 1)].L == k.max_layers;
+    const double rest = total - batch_shapes(k.n)[0].work * layers[c];
+    double best = 0.0;
+    for (const BatchShape &s : batch_shapes(k.n)) {
+      // clusters do not straddle GPCs: of 148 SMs 144 hold clusters of 4 and 8, 112 of 16
+      const int usable = sms * (s.shape.log_ctas < 2 ? 148 : s.shape.log_ctas < 4 ? 144 : 112) / 148;
+      const int clusters = std::max(1, usable >> s.shape.log_ctas);
+      const double busy = s.work * clusters / sms;
+      double own = s.latency * k.max_layers;
+      if (even && k.count < clusters)
+        own = std::max(own, (s.latency + (busy - s.latency) * k.count / clusters) * k.max_layers);
+      else if (even)
+        own = std::max(own, (k.count + clusters - 1) / clusters * busy * k.max_layers);
+      const double t = std::max((rest + s.work * layers[c]) / sms, own) + 0.25 * s.latency * k.max_layers;
+      if (best != 0.0 && t >= best) continue;
+      best = t;
+      k.shape = s.shape;
+    }
+  }
+}
 
 // The circuits by qubit count (largest first) and depth (deepest first); false
 // where the device does not hold a cluster of some class.
@@ -1663,14 +1719,10 @@ bool batch_classes(rsv_batch *Bt, const std::vector<BatchCircuit> &circ) {
   for (int c : order) {
     const BatchCircuit &C = circ[static_cast<size_t>(c)];
     if (Bt->classes.empty() || Bt->classes.back().n != C.n) {
-      int &fit = Bt->fits[C.n];  // asked once a qubit count, for the deepest circuits
-      if (fit == 0) check(cluster_capacity(C.n, batch_shape_for(C.n), kBatchMaxLayers, &fit), "cluster capacity");
-      if (fit < 1) return false;
       rsv_batch::Class k{};
       k.n = C.n;
       k.first = static_cast<int>(items.size());
       k.max_layers = C.L;
-      k.shape = batch_shape_for(C.n);
       Bt->classes.push_back(k);
     }
     ++Bt->classes.back().count;
@@ -1681,22 +1733,25 @@ bool batch_classes(rsv_batch *Bt, const std::vector<BatchCircuit> &circ) {
     it.h = C.h;
     items.push_back(it);
   }
-  // checkpoints for as many clusters of each class as the device holds
+  batch_choose_shapes(Bt->classes, items, Bt->sms);
+  // the tiled classes' vectors, for as many clusters as the device holds
   size_t values = 0;
   for (auto &k : Bt->classes) {
-    k.clusters = std::min(k.count, Bt->fits[k.n]);
-    const size_t v = cluster_checkpoint_values(k.n, k.shape, k.max_layers) * static_cast<size_t>(k.clusters);
-    if ((values + v) * sizeof(double2) > kBatchCheckpointBytes) k.shape.checkpoints = false;
-    if (!k.shape.checkpoints) continue;
-    k.checkpoint = values;
+    int &fit = Bt->fits[k.n][k.shape.log_ctas];  // asked once a shape, for the deepest circuits
+    if (fit == 0) check(cluster_capacity(k.n, k.shape, kBatchMaxLayers, &fit), "cluster capacity");
+    if (fit < 1) return false;
+    k.clusters = std::min(k.count, fit);
+    const size_t v = cluster_memory_values(k.n, k.shape, k.max_layers) * static_cast<size_t>(k.clusters);
+    if (!k.shape.tiled) continue;
+    k.vectors = values;
     values += v;
   }
   try {
-    if (Bt->d_checkpoints.count < values) Bt->d_checkpoints.alloc(values);
+    if (Bt->d_vectors.count < values) Bt->d_vectors.alloc(values);
   } catch (const Error &e) {
     if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
-    cudaGetLastError();  // clear the allocation failure; psi is un-computed
-    for (auto &k : Bt->classes) k.shape.checkpoints = false;
+    cudaGetLastError();  // clear the allocation failure; the persistent kernel has its scratch
+    return false;
   }
   if (Bt->d_counters.p == nullptr) Bt->d_counters.alloc(kBatchMaxQubits + 1);
   while (Bt->side.size() + 1 < Bt->classes.size()) {
@@ -1771,10 +1826,10 @@ void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *
       A.n = c.n;
       A.shape = c.shape;
       A.count = c.count;
-      if (c.shape.checkpoints) {
+      if (c.shape.tiled) {
         A.clusters = c.clusters;
         A.counter = Bt->d_counters.p + c.n;
-        A.checkpoints = Bt->d_checkpoints.p + c.checkpoint;
+        A.memory = Bt->d_vectors.p + c.vectors;
       }
       A.items = Bt->d_items.p + c.first;
       A.max_layers = c.max_layers;
@@ -2037,14 +2092,17 @@ bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 16 && L == 5)
 // CTA (n = 9 23.6 us, 8 a thread 24.8, 16 a thread 47), 10 and 11 qubits 8 a
 // thread (31 and 51 us; 4 a thread 35 and 55), 12 and 13 on 8 CTAs (64 and 86
 // us; on one or two 90 and 180), then 16 CTAs (14 qubits 120 us against 137 on
-// 8).  Checkpoints pay from 15 qubits on, where un-computing psi means moving it
-// between CTAs (15 qubits 163 us against 170, 16 qubits 258 against 293; 14
-// qubits 123 against 120, 12 qubits 72 against 64).
+// 8).  Checkpoints pay where un-computing psi means moving it between CTAs (15
+// qubits 163 us against 170; 14 qubits 123 against 120, 12 qubits 72 against
+// 64), and with 16 qubits the exchanges cost more than passing the state through
+// memory, tiled (184 us against 258; 15 qubits 167 against 163, 14 qubits 167
+// against 123).
 ClusterShape cluster_shape_for(int n) {
   if (n <= 9) return {0, 2, false};
   if (n <= 11) return {0, 3, false};
   if (n <= 13) return {3, 3, false};
-  return {4, 4, n >= 15};
+  if (n <= 15) return {4, 4, n == 15};
+  return {4, 4, false, true};
 }
 
 // What runs a backend's calls.  A caller that chose a backward schedule, fewer
@@ -2104,7 +2162,7 @@ void setup_plan(rsv_backend *B, int mode) {
   if (B->path == Path::kRing)
     values = 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs;
   else if (B->path == Path::kCluster)
-    values = cluster_checkpoint_values(B->n, B->cluster_shape, B->L) + 2 * B->state_len;
+    values = cluster_memory_values(B->n, B->cluster_shape, B->L) + 2 * B->state_len;
   if (values > static_cast<size_t>(pl.num_bufs) * B->state_len) {
     try {
       B->states.alloc(values);
@@ -2747,7 +2805,7 @@ rsv_status rsv_describe_backend(rsv_backend *B, char *buf, size_t buf_size, size
        << " tma_passes=" << B->tma_passes;
     if (B->path == Path::kRing) os << " ring_contraction (the plan below is not used)";
     if (B->path == Path::kCluster)
-      os << " cluster_resident: " << (1 << B->cluster_shape.log_ctas) << " CTAs x " << (1 << B->cluster_shape.register_bits) << " amplitudes (the plan below is not used)";
+      os << " cluster_resident: " << (1 << B->cluster_shape.log_ctas) << " CTAs x " << (1 << B->cluster_shape.register_bits) << " amplitudes" << (B->cluster_shape.tiled ? ", tiled" : "") << " (the plan below is not used)";
     if (B->energy_fuse_pass >= 0)
       os << " fused_energy: backward pass " << B->energy_fuse_pass << " applies "
          << kTmaNumEnergyMasks << " field terms,"

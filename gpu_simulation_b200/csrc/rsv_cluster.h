@@ -19,19 +19,21 @@ struct ClusterItem {
 };
 
 // How a launch spreads a circuit: 2^log_ctas CTAs, 2^register_bits amplitudes a
-// thread; with checkpoints the backward reads psi from memory.
+// thread; with checkpoints the backward reads psi from memory.  Tiled: psi and
+// lambda are in memory, and the CTAs work through them tile by tile.
 struct ClusterShape {
   int log_ctas, register_bits;
   bool checkpoints;
+  bool tiled = false;
 };
 
 struct ClusterArgs {
   int n;
   ClusterShape shape;
   int count;                   // circuits
-  int clusters;                // with a counter: clusters that take them in turn
-  int *counter;                // or null: one cluster a circuit
-  double2 *checkpoints;        // clusters * cluster_checkpoint_values(n, shape, max_layers)
+  int clusters;                // with a counter (tiled): clusters that take them in turn
+  int *counter;                // 0 at the launch, or null: one cluster a circuit
+  double2 *memory;             // clusters * cluster_memory_values(n, shape, max_layers)
   const ClusterItem *items;    // [count], or null: the one circuit `item`
   ClusterItem item;
   int max_layers;              // largest L of the circuits
@@ -41,16 +43,22 @@ struct ClusterArgs {
   double *energy_out;          // or null
   double *grad_out;            // or null: no backward
   // One circuit only: the forward call leaves psi (without checkpoints) and
-  // H psi here, and with `resume` a later call starts from them (and the
+  // H psi here (tiled: in `memory`), and with `resume` a later call starts from them (and the
   // checkpoints) and runs the backward alone.
   double2 *psi, *lam;
   int resume;
 };
 
 bool cluster_shape_built(int n, ClusterShape h);
-size_t cluster_checkpoint_values(int n, ClusterShape h, int max_layers);
+// Global memory of a cluster: psi's checkpoints, or a tiled circuit's vectors.
+size_t cluster_memory_values(int n, ClusterShape h, int max_layers);
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s);
 // Clusters of that shape that fit the device at once (0: none).
 cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *clusters);
+
+// Tiled circuits (rsv_tiles.cu); the functions above go there.
+bool tile_shape_built(int n, ClusterShape h);
+cudaError_t launch_tiles(const ClusterArgs &A, cudaStream_t s);
+cudaError_t tile_capacity(int n, ClusterShape h, int max_layers, int *clusters);
 
 }  // namespace rsv
