@@ -899,7 +899,8 @@ struct rsv_backend {
       mps_gf;
   // what runs a call: the tile passes, the contraction along the ring
   // (rsv_ring.cu; its kept components lie in the state buffers) or the
-  // cluster-resident state (rsv_cluster.cu); and the field of the last forward
+  // cluster-resident state (rsv_cluster.cu, rsv_tiles.cu, rsv_grid.cu); and the
+  // field of the last forward
   rsv::Path path = rsv::Path::kPasses;
   rsv::ClusterShape cluster_shape{0, 4, true};
   double forward_field = 0.0;
@@ -2096,13 +2097,15 @@ bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 16 && L == 5)
 // qubits 163 us against 170; 14 qubits 123 against 120, 12 qubits 72 against
 // 64), and with 16 qubits the exchanges cost more than passing the state through
 // memory, tiled (184 us against 258; 15 qubits 167 against 163, 14 qubits 167
-// against 123).
+// against 123).  From 17 qubits on that takes the whole device: L = 6 and 16, us,
+// against the tile passes: n = 17 173 and 453 (226, 740), n = 18 176 and 452 (228,
+// 744), n = 19 185 and 481 (236, 784), n = 20 319 and 822 (337, 1115).
 ClusterShape cluster_shape_for(int n) {
   if (n <= 9) return {0, 2, false};
   if (n <= 11) return {0, 3, false};
   if (n <= 13) return {3, 3, false};
   if (n <= 15) return {4, 4, n == 15};
-  return {4, 4, false, true};
+  return {n <= kClusterMaxQubits ? 4 : 0, 4, false, true};  // from 17 on one CTA a SM
 }
 
 // What runs a backend's calls.  A caller that chose a backward schedule, fewer
@@ -2113,7 +2116,7 @@ Path choose_path(rsv_backend *B, int mode) {
                         B->kernel_flags == (RSV_KERNELS_TMA | RSV_KERNELS_FUSED_ENERGY) && B->force_c == 0;
   if (!defaults || B->dense || B->gate_level) return Path::kPasses;
   if (ring_rule(B->n, B->L)) return Path::kRing;
-  if (B->n > kClusterMaxQubits || B->L > kClusterMaxLayers) return Path::kPasses;
+  if (B->n > kGridMaxQubits || B->L > kClusterMaxLayers) return Path::kPasses;
   B->cluster_shape = cluster_shape_for(B->n);
   int clusters = 0;
   if (cluster_capacity(B->n, B->cluster_shape, B->L, &clusters) != cudaSuccess)
@@ -2805,7 +2808,10 @@ rsv_status rsv_describe_backend(rsv_backend *B, char *buf, size_t buf_size, size
        << " tma_passes=" << B->tma_passes;
     if (B->path == Path::kRing) os << " ring_contraction (the plan below is not used)";
     if (B->path == Path::kCluster)
-      os << " cluster_resident: " << (1 << B->cluster_shape.log_ctas) << " CTAs x " << (1 << B->cluster_shape.register_bits) << " amplitudes" << (B->cluster_shape.tiled ? ", tiled" : "") << " (the plan below is not used)";
+      os << (B->n > kClusterMaxQubits ? " whole_device: a CTA a SM"
+                                      : " cluster_resident: " + std::to_string(1 << B->cluster_shape.log_ctas) + " CTAs")
+         << " x " << (1 << B->cluster_shape.register_bits) << " amplitudes" << (B->cluster_shape.tiled ? ", tiled" : "")
+         << " (the plan below is not used)";
     if (B->energy_fuse_pass >= 0)
       os << " fused_energy: backward pass " << B->energy_fuse_pass << " applies "
          << kTmaNumEnergyMasks << " field terms,"

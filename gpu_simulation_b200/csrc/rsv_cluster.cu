@@ -528,12 +528,14 @@ bool with_shape(int n, ClusterShape h, F &&f) {
 }  // namespace
 
 bool cluster_shape_built(int n, ClusterShape h) {
+  if (n > kClusterMaxQubits) return h.tiled && n <= kGridMaxQubits;
   if (h.tiled) return tile_shape_built(n, h);
   return with_shape(n, h, [](auto) {});
 }
 
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s) {
   if (A.count < 1) return cudaSuccess;
+  if (A.n > kClusterMaxQubits) return launch_grid(A, s);
   if (A.shape.tiled) return launch_tiles(A, s);
   cudaError_t e = cudaErrorInvalidValue;
   with_shape(A.n, A.shape, [&](auto shape) { e = decltype(shape)::launch(A, s); });
@@ -542,6 +544,7 @@ cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s) {
 
 cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *clusters) {
   *clusters = 0;
+  if (n > kClusterMaxQubits) return grid_capacity(n, max_layers, clusters);
   if (h.tiled) return tile_capacity(n, h, max_layers, clusters);
   cudaError_t e = cudaSuccess;
   with_shape(n, h, [&](auto shape) { e = decltype(shape)::capacity(max_layers, clusters); });
@@ -549,6 +552,7 @@ cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *cluster
 }
 
 size_t cluster_memory_values(int n, ClusterShape h, int max_layers) {
+  if (n > kClusterMaxQubits) return grid_memory_values(n, max_layers);
   if (h.tiled) return size_t{4} << n;
   size_t v = 0;
   with_shape(n, h, [&](auto shape) { v = decltype(shape)::memory_values(max_layers); });

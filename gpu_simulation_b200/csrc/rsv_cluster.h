@@ -61,4 +61,11 @@ bool tile_shape_built(int n, ClusterShape h);
 cudaError_t launch_tiles(const ClusterArgs &A, cudaStream_t s);
 cudaError_t tile_capacity(int n, ClusterShape h, int max_layers, int *clusters);
 
+// One circuit of more than kClusterMaxQubits (rsv_grid.cu): tiled on the whole
+// device; the functions above go there.
+constexpr int kGridMaxQubits = 20;
+size_t grid_memory_values(int n, int max_layers);
+cudaError_t launch_grid(const ClusterArgs &A, cudaStream_t s);
+cudaError_t grid_capacity(int n, int max_layers, int *circuits);
+
 }  // namespace rsv

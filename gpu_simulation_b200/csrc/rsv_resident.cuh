@@ -21,13 +21,14 @@ constexpr int kRecPhi = 16, kRecTotal = 20, kRecLane = 21;
 
 #define RSV_HD __host__ __device__ __forceinline__ constexpr
 
-RSV_HD unsigned ring_map(unsigned x, int n) {  // P (rsv_device.cuh, at most 16 bits)
+RSV_HD unsigned ring_map(unsigned x, int n) {  // P (rsv_device.cuh, at most 32 bits)
   const unsigned mask = (1u << n) - 1;
   unsigned p = x & mask;
   p ^= p << 1;
   p ^= p << 2;
   p ^= p << 4;
   p ^= p << 8;
+  if (n > 16) p ^= p << 16;
   p &= mask;
   return (x & ~mask) | (p & ~1u) | (((p >> (n - 1)) ^ x) & 1u);
 }
