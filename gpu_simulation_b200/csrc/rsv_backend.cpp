@@ -1114,8 +1114,9 @@ void run_forward(rsv_backend *B, cudaStream_t st) {
 // a plan with such a pass.
 bool fused_energy(const rsv_backend *B, bool grad) { return grad && B->energy_fuse_pass >= 0; }
 
-void run_energy(rsv_backend *B, cudaStream_t st, bool fused) {
-  const double bytes = 2.0 * 16.0 * static_cast<double>(u64{1} << B->n);
+// store: lambda = H psi is needed.
+void run_energy(rsv_backend *B, cudaStream_t st, bool fused, bool store = true) {
+  const double bytes = (store ? 2.0 : 1.0) * 16.0 * static_cast<double>(u64{1} << B->n);
   if (fused) {
     timed(B, st, 2, bytes, [&] {
       check(launch_energy_masks(state_buf(B, B->plan.chi_buf), state_buf(B, B->plan.mu_buf), B->n, B->field,
@@ -1126,7 +1127,7 @@ void run_energy(rsv_backend *B, cudaStream_t st, bool fused) {
     return;
   }
   timed(B, st, 2, bytes, [&] {
-    check(launch_energy(state_buf(B, B->plan.chi_buf), state_buf(B, B->plan.mu_buf), B->n, B->field,
+    check(launch_energy(state_buf(B, B->plan.chi_buf), store ? state_buf(B, B->plan.mu_buf) : nullptr, B->n, B->field,
                         u64{1} << B->n, B->energy_partials.p, B->energy_grid, B->sms, st),
           "energy launch");
   }, energy_kernel_count(B->n));
@@ -1179,11 +1180,12 @@ void run_backward(rsv_backend *B, cudaStream_t st, bool fused) {
 }
 
 void run_finalize(rsv_backend *B, bool grad, double *energy_out, double *grad_out,
-                  cudaStream_t st, bool fused = false) {
+                  cudaStream_t st, bool fused = false, bool stored = true) {
   FinalizeParams F{};
   F.n = B->n;
   F.L = B->L;
-  F.num_energy_partials = B->energy_grid + (fused ? B->energy_fuse_grid + B->energy_defer_grid : 0);
+  F.num_energy_partials = stored ? B->energy_grid + (fused ? B->energy_fuse_grid + B->energy_defer_grid : 0)
+                                 : energy_partial_count(B->n, B->sms);
   F.phi_alt_layer = -1;
   if (B->energy_defer_pass >= 0) {
     F.phi_alt_layer = B->L - 1;
@@ -1385,9 +1387,11 @@ void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_o
   launch_prep(B, st);
   run_forward(B, st);
   const bool fused = fused_energy(B, grad);
-  run_energy(B, st, fused);
+  // (a caller's workspace holds the partials of the stored form only)
+  const bool store = grad || keep || B->energy_partials.count < static_cast<size_t>(energy_partial_count(B->n, B->sms));
+  run_energy(B, st, fused, store);
   if (grad) run_backward(B, st, fused);
-  run_finalize(B, grad, energy_out, grad_out, st, fused);
+  run_finalize(B, grad, energy_out, grad_out, st, fused, store);
 }
 
 // After a synchronised call: a NaN energy from a backend with TMA passes may

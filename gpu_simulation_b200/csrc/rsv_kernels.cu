@@ -194,7 +194,9 @@ struct EnergyMasks {
 // grid-stride part: the K masks of M, plus mu_in (the tile kernel's part,
 // diagonal included) when given, else the diagonal.  K is a template
 // parameter so that all K partner loads of an amplitude are issued before
-// the first is used.
+// the first is used.  Without `mu` (an energy that no gradient follows) nothing is
+// stored, and each kernel adds its own terms' energy: L = 6, n = 23 772 -> 751 us,
+// n = 25 2767 -> 2703.
 template <int K, int THREADS>
 __global__ void __launch_bounds__(THREADS) energy_kernel(const double2 *__restrict__ chi,
                                                                  double2 *__restrict__ mu, int n,
@@ -214,14 +216,16 @@ __global__ void __launch_bounds__(THREADS) energy_kernel(const double2 *__restri
       x.y += t.y;
     }
     double2 m;
-    if (with_mu_in) {
+    if (with_mu_in && mu == nullptr) {
+      m = make_double2(-field * x.x, -field * x.y);
+    } else if (with_mu_in) {
       const double2 mi = mu[i];
       m = make_double2(fma(-field, x.x, mi.x), fma(-field, x.y, mi.y));
     } else {
       const double d = diag_after_ring(i, n);
       m = make_double2(fma(d, c.x, -field * x.x), fma(d, c.y, -field * x.y));
     }
-    mu[i] = m;
+    if (mu != nullptr) mu[i] = m;
     e += fma(c.x, m.x, c.y * m.y);
   }
   e = warp_sum(e);
@@ -283,7 +287,9 @@ __device__ __forceinline__ u64 energy_tile_index(u64 cbase, int tau, int hs) {
 
 __global__ void __launch_bounds__(kEnergyTileThreads) energy_tile_kernel(const double2 *__restrict__ chi,
                                                                           double2 *__restrict__ mu,
-                                                                          const EnergyTile T) {
+                                                                          const EnergyTile T, double *__restrict__ partials) {
+  __shared__ double red[kEnergyTileThreads / 32];
+  double e = 0.0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2 *tile = reinterpret_cast<double2 *>(smem_raw);
   constexpr int kPer = (1 << kEnergyTileBits) / kEnergyTileThreads;
@@ -314,9 +320,24 @@ __global__ void __launch_bounds__(kEnergyTileThreads) energy_tile_kernel(const d
         x.y += v.y;
       }
       const double d = diag_after_ring(p, T.n);
-      __stcg(&mu[p], make_double2(fma(d, c.x, -T.field * x.x), fma(d, c.y, -T.field * x.y)));
+      const double2 m = make_double2(fma(d, c.x, -T.field * x.x), fma(d, c.y, -T.field * x.y));
+      if (mu != nullptr) __stcg(&mu[p], m);
+      else e += fma(c.x, m.x, c.y * m.y);
     }
   }
+  if (mu != nullptr) return;
+  e = warp_sum(e);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int i = 0; i < kEnergyTileThreads / 32; ++i) s += red[i];
+    partials[blockIdx.x] = s;
+  }
+}
+
+int energy_tile_grid(int n, int sms) {
+  return static_cast<int>(std::min<u64>(u64{1} << (n - kEnergyTileBits), static_cast<u64>(std::max(1, sms)) * 3));
 }
 
 // ------------------------------------------------------------------------
@@ -457,8 +478,7 @@ cudaError_t launch_energy(const double2 *chi, double2 *mu, int n, double field, 
     const cudaError_t e = set_smem_limit_once(energy_tile_kernel, kEnergyTileSmem, configured);
     if (e != cudaSuccess) return e;
   }
-  const int tgrid = static_cast<int>(std::min<u64>(T.num_tiles, static_cast<u64>(std::max(1, sms)) * 3));
-  energy_tile_kernel<<<tgrid, kEnergyTileThreads, kEnergyTileSmem, s>>>(chi, mu, T);
+  energy_tile_kernel<<<energy_tile_grid(n, sms), kEnergyTileThreads, kEnergyTileSmem, s>>>(chi, mu, T, partials + grid);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_energy_k<1>(count, grid, s, chi, mu, n, field, size, M, 1, partials);
@@ -476,6 +496,10 @@ cudaError_t launch_energy_masks(const double2 *chi, double2 *mu, int n, double f
 int energy_split_qubits() { return kEnergySplitQubits; }
 
 int energy_kernel_count(int n) { return n < kEnergySplitQubits ? 1 : 2; }
+
+int energy_partial_count(int n, int sms) {
+  return energy_grid_size(n, sms) + (n < kEnergySplitQubits ? 0 : energy_tile_grid(n, sms));
+}
 
 int energy_grid_size(int n, int sms) {
   const u64 size = u64{1} << n;

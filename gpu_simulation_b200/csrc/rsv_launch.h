@@ -40,7 +40,8 @@ cudaError_t launch_pass(const PassParams &P, bool bwd, int grid, cudaStream_t s)
 // backward pass on an 11-bit half tile (rsv_pass_half.cu)
 cudaError_t launch_bwd_half(const PassParams &P, int grid, cudaStream_t s);
 // mu = (P^T H P) chi and per-CTA energy partials ([grid]); for large n a
-// shared-memory tile kernel takes the masks on the top index bits first
+// shared-memory tile kernel takes the masks on the top index bits first.  mu may
+// be null: the energy alone, with energy_partial_count partials
 cudaError_t launch_energy(const double2 *chi, double2 *mu, int n, double field,
                           unsigned long long size, double *partials, int grid, int sms, cudaStream_t s);
 // mu = (diagonal - field * sum over the given index masks) chi, with per-CTA
@@ -65,6 +66,7 @@ int energy_split_qubits();
 int energy_kernel_count(int n);
 // CTAs of the energy's grid-stride kernel (= its number of partials)
 int energy_grid_size(int n, int sms);
+int energy_partial_count(int n, int sms);
 cudaError_t launch_finalize(const FinalizeParams &F, cudaStream_t s);
 // layer-0 gradients in one read of lambda (n >= 13), and their final reduction
 // into grad_out[0 .. 2n)
