@@ -1280,6 +1280,7 @@ ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_
   A.n = B->n;
   A.shape = B->cluster_shape;
   A.memory = B->states.p;
+  if (B->n > kClusterMaxQubits) A.counter = B->pipeline_err.p;
   A.count = 1;
   A.item.L = A.max_layers = B->L;
   A.item.h = B->forward_field;
@@ -1398,12 +1399,12 @@ void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_o
 // come from a pipeline wait that gave up (finalize_kernel writes NaN then);
 // report it as an error and clear the flag.
 void check_pipeline(rsv_backend *B, double energy) {
-  if (B->tma_passes == 0 || !std::isnan(energy)) return;
+  if ((B->tma_passes == 0 && B->path != Path::kCluster) || !std::isnan(energy)) return;
   int flag = 0;
   check(cudaMemcpy(&flag, B->pipeline_err.p, sizeof(int), cudaMemcpyDeviceToHost), "pipeline flag read");
   if (flag == 0) return;
   check(cudaMemset(B->pipeline_err.p, 0, sizeof(int)), "pipeline flag clear");
-  throw Error(RSV_ERR_CUDA, "a TMA backward pass gave up waiting for its pipeline (flag " +
+  throw Error(RSV_ERR_CUDA, "a kernel gave up waiting for its pipeline or its other blocks (flag " +
                                 std::to_string(flag) + "); the results of this call are void");
 }
 

@@ -32,7 +32,8 @@ struct ClusterArgs {
   ClusterShape shape;
   int count;                   // circuits
   int clusters;                // with a counter (tiled): clusters that take them in turn
-  int *counter;                // 0 at the launch, or null: one cluster a circuit
+  int *counter;                // 0 at the launch, or null: one cluster a circuit; whole device: set where a
+                               // CTA gave up waiting for the others
   double2 *memory;             // clusters * cluster_memory_values(n, shape, max_layers)
   const ClusterItem *items;    // [count], or null: the one circuit `item`
   ClusterItem item;

@@ -14,7 +14,8 @@
 // with the first three layers as matrix products.  A layer now takes 28 us from
 // 17 to 19 qubits, a tile or less a CTA, of which the four barriers are about 8;
 // with 20 qubits 50 us: 108 of 148 CTAs have a second tile, which the others wait
-// for.  Energy and gradient at L = 8: n = 17 330 -> 230 us, n = 18 331 -> 229, n =
+// for (issuing its loads ahead, as rsv_tiles.cu does, made L = 8 456 us instead of
+// 422).  Energy and gradient at L = 8: n = 17 330 -> 230 us, n = 18 331 -> 229, n =
 // 19 349 -> 246, n = 20 493 -> 422.
 #include <cuda_runtime.h>
 
@@ -42,6 +43,7 @@ constexpr int kGridRec = 48, kGridHigh = 4, kGridPhi = 8, kGridTotal = 12, kGrid
 // How often a CTA looks whether the others have arrived (about a second), then
 // it gives up for all of them.
 constexpr int kGridSpins = 1 << 21;
+constexpr int kGridLost = 1 << 8;  // what the caller's flag then holds
 
 // Behind the four vectors: records [layer][value][CTA], energies [CTA], then
 struct GridState {
@@ -447,6 +449,7 @@ template <int n>
 __global__ void __launch_bounds__(256, 1) grid_circuit_kernel(const __grid_constant__ ClusterArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   if (run_grid<n>(A, smem)) return;
+  if (threadIdx.x == 0) atomicMax(A.counter, kGridLost);
   const double nan = __longlong_as_double(0x7ff8000000000000ll);  // a CTA did not arrive
   if (A.energy_out && blockIdx.x == 0 && threadIdx.x == 0) A.energy_out[A.item.index] = nan;
   if (A.grad_out)
@@ -484,7 +487,7 @@ struct GridShape {
     int count = 0;
     cudaError_t e = ctas(A.max_layers, &count);
     if (e != cudaSuccess) return e;
-    if (count < 1 || A.count != 1 || A.items != nullptr) return cudaErrorInvalidValue;
+    if (count < 1 || A.count != 1 || A.items != nullptr || A.counter == nullptr) return cudaErrorInvalidValue;
     void *state = reinterpret_cast<double *>(A.memory + (size_t{4} << n)) + grid_doubles(A.max_layers);
     if ((e = cudaMemsetAsync(state, 0, sizeof(GridState), s)) != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};

@@ -322,6 +322,17 @@ __device__ __forceinline__ Tables build_tables(const double *params, const doubl
   return T;
 }
 
+// A thread's amplitudes of the next tile on their way into its own 16 slots of a
+// buffer ([register][thread]); only that thread reads them.
+__device__ __forceinline__ void fetch(unsigned char *buf, int r, const double2 *from) {
+  const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(buf)) + ((r << 8) + threadIdx.x) * 16;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+}
+__device__ __forceinline__ void fetched() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ double2 take(const unsigned char *buf, int r) {
+  return reinterpret_cast<const double2 *>(buf)[(r << 8) + threadIdx.x];
+}
+
 template <bool V>
 struct Flag {
   static constexpr bool value = V;
