@@ -1,11 +1,13 @@
 """Batched ring-Ising circuits: thousands of independent (n, L, h) circuits per
-kernel launch (include/rsv.h ``rsv_batch_*``).
+call (include/rsv.h ``rsv_batch_*``).
 
 The reference evaluates one circuit per ``RingIsingCudaBackend`` object
 (``cpp/ising_cuda_backend.hpp:22-49``); a batch there is a Python loop over
-backends.  Here one persistent kernel takes the whole list: one CTA per
-circuit at a time, circuits handed out longest first from an atomic counter,
-every circuit running the pass plan the single-circuit engine would run.
+backends.  Here a launch per qubit count takes all circuits of that size, states
+in the registers of one CTA up to 12 qubits and passed through 1 to 16 CTAs in
+tiles above; or, where slots or a cluster size are given, one persistent kernel
+takes the whole list, circuits handed out longest first from an atomic counter,
+every circuit running the pass plan of the single-circuit engine.
 
 Packed layout: circuit ``c`` owns ``params[off[c] : off[c] + 2*n_c*L_c]`` with
 the per-circuit layout ``(L, n, 2)`` flattened; gradients use the same packing.
