@@ -125,26 +125,33 @@ Tile antipodal_tile(int n) {
 // c is chosen to minimise the number of passes, then -- with wide_last, for
 // the forward tiles of the checkpoint schedule -- to leave the last tile at
 // most 8 gated wires (at least 4 contiguous low bits: its backward half tile
-// then runs on the tensor-copy kernel and takes the fused field terms), then
-// maximised (longer DRAM segments), unless force_c (2..10) fixes it (the
-// autotuner's candidates).  Returns the tiles (gates on the split wires).
+// then runs on the tensor-copy kernel and takes the fused field terms) and then
+// to be 4 where the last tile keeps at least 5 (the other tiles' half tiles then
+// have runs of 3 and 8 bits, few enough for that kernel too: energy and gradient, n =
+// 25, L = 7 8.47 ms against 8.76 with 5 bits, n = 26, L = 6 12.96 against 13.34; with
+// fewer than 5 the last one's run is too long for the field terms), then maximised
+// (longer DRAM segments), unless force_c (2..10) fixes it (the autotuner's
+// candidates).  Returns the tiles (gates on the split wires).
 std::vector<Tile> high_tiles(int n, int lo, int min_c = 2, int force_c = 0, bool wide_last = false) {
   std::vector<Tile> out;
   const int m = n - lo;
   if (m <= 0) return out;
   int best_c = min_c, best_passes = 1 << 30;
-  bool best_wide = false;
+  bool best_wide = false, best_four = false;
   for (int c = min_c; c <= 10; ++c) {
     const int g = 12 - c;
     if (c > lo) break;  // contiguity bits must lie below the gated wires
     const int passes = (m + g - 1) / g;
     const bool wide = wide_last && m - (passes - 1) * g <= 8;
+    const bool four = wide_last && passes > 1 && c == 4 && m - (passes - 1) * g >= 5;
     const bool better = passes < best_passes ||
-                        (passes == best_passes && (wide != best_wide ? wide : c > best_c));
+                        (passes == best_passes &&
+                         (wide != best_wide ? wide : four != best_four ? four : c > best_c));
     if (better) {
       best_passes = passes;
       best_c = c;
       best_wide = wide;
+      best_four = four;
     }
   }
   if (force_c >= min_c && force_c <= std::min(10, lo)) best_c = force_c;
