@@ -157,6 +157,15 @@ def load_library() -> ctypes.CDLL:
     return lib
 
 
+def raw_stream(device_index: int) -> int:
+    """The handle of torch's current stream on a device.  Without the Stream
+    object that torch.cuda.current_stream builds around it (2.2 us against 0.1,
+    of a small circuit's 15 us call)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(device_index)
+
+
 def check(status: int) -> None:
     """Raise ValueError / EngineError for a non-zero rsv_status."""
     if status == RSV_OK:

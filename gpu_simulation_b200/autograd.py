@@ -16,7 +16,7 @@ import ctypes
 
 import torch
 
-from ._lib import RSV_ERR_STALE_STATE, check
+from ._lib import RSV_ERR_STALE_STATE, check, raw_stream
 from .engine import Engine
 
 
@@ -28,29 +28,28 @@ class RingIsingEnergy(torch.autograd.Function):
         flat = params.detach().reshape(-1).contiguous()
         if flat.numel() != engine.num_params:
             raise ValueError(f"expected {engine.num_params} parameters, got {flat.numel()}")
-        energy = torch.empty(1, dtype=torch.float64, device=params.device)
-        stream = torch.cuda.current_stream(params.device)
+        energy = torch.empty((), dtype=torch.float64, device=params.device)
         gen = ctypes.c_ulonglong()
         check(engine._lib.rsv_forward_device(engine._h, flat.data_ptr(), flat.numel(),
-                                             energy.data_ptr(), ctypes.byref(gen), stream.cuda_stream))
+                                             energy.data_ptr(), ctypes.byref(gen),
+                                             raw_stream(params.get_device())))
         ctx.engine = engine
         ctx.generation = gen.value
         ctx.shape = params.shape
         ctx.save_for_backward(flat)
-        return energy.reshape(())
+        return energy
 
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):
         (flat,) = ctx.saved_tensors
         engine: Engine = ctx.engine
         grad = torch.empty_like(flat)
-        stream = torch.cuda.current_stream(flat.device)
         status = engine._lib.rsv_backward_device(engine._h, ctx.generation, grad.data_ptr(),
-                                                 stream.cuda_stream)
+                                                 raw_stream(flat.get_device()))
         if status == RSV_ERR_STALE_STATE:
             # the engine's buffers were reused by another call: recompute
             scratch = torch.empty(1, dtype=torch.float64, device=flat.device)
-            engine.energy_and_grad_device(flat, scratch, grad, stream)
+            engine.energy_and_grad_device(flat, scratch, grad)
         else:
             check(status)  # any other failure is raised, never retried
         return (grad * grad_output).reshape(ctx.shape), None

@@ -12,7 +12,7 @@ import ctypes
 
 import numpy as np
 
-from ._lib import check, load_library
+from ._lib import check, load_library, raw_stream
 
 
 class Engine:
@@ -90,10 +90,10 @@ class Engine:
             raise ValueError("num_params does not match the circuit.")
         if grad_out is not None and grad_out.numel() != self.num_params:
             raise ValueError("grad_out does not match the circuit.")
-        s = stream if stream is not None else torch.cuda.current_stream(params.device)
+        s = stream.cuda_stream if stream is not None else raw_stream(params.get_device())
         check(self._lib.rsv_energy_and_grad_device(
             self._h, params.data_ptr(), params.numel(), energy_out.data_ptr(),
-            grad_out.data_ptr() if grad_out is not None else None, s.cuda_stream))
+            grad_out.data_ptr() if grad_out is not None else None, s))
 
     def benchmark_forward_graph(self, params, repeats: int = 100) -> dict:
         flat = self._flat(params)

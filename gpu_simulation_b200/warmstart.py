@@ -21,7 +21,7 @@ import time
 
 import numpy as np
 
-from ._lib import check, load_library
+from ._lib import check, load_library, raw_stream
 from .batch import BatchEngine
 
 WIDTHS = (3, 256, 256, 192)
@@ -92,21 +92,20 @@ class WarmStartMLP:
         self._lib = load_library()
         self.widths = tuple(int(w) for w in widths)
         self._w_arr = np.asarray(self.widths, dtype=np.int32)
+        self._w_ptr = self._w_arr.ctypes.data
         self.num_layers = len(self.widths) - 1
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else device
-        n_w = self._lib.rsv_mlp_num_weights(self.num_layers, self._w_arr.ctypes.data)
+        n_w = self._lib.rsv_mlp_num_weights(self.num_layers, self._w_ptr)
         self.weights = torch.from_numpy(init_weights(self.widths, seed)).to(self.device)
         assert self.weights.numel() == n_w
 
     def _stream(self):
-        import torch
-
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return raw_stream(self.weights.get_device())
 
     def _work(self, batch: int):
         import torch
 
-        nw = self._lib.rsv_mlp_work_floats(self.num_layers, self._w_arr.ctypes.data, batch)
+        nw = self._lib.rsv_mlp_work_floats(self.num_layers, self._w_ptr, batch)
         return torch.empty(max(1, nw), dtype=torch.float32, device=self.device)
 
     def forward(self, x, work=None):
@@ -116,7 +115,7 @@ class WarmStartMLP:
         x = x.to(self.device, torch.float32).contiguous()
         out = torch.empty((x.shape[0], self.widths[-1]), dtype=torch.float32, device=self.device)
         work = self._work(x.shape[0]) if work is None else work
-        check(self._lib.rsv_mlp_forward(self.num_layers, self._w_arr.ctypes.data, self.weights.data_ptr(),
+        check(self._lib.rsv_mlp_forward(self.num_layers, self._w_ptr, self.weights.data_ptr(),
                                         x.shape[0], x.data_ptr(), out.data_ptr(), work.data_ptr(),
                                         self._stream()))
         return out
@@ -127,20 +126,21 @@ class WarmStartMLP:
 
         x = x.to(self.device, torch.float32).contiguous()
         target = target.to(self.device, torch.float32).contiguous()
-        work = self._work(x.shape[0])
-        out = self.forward(x, work)
-        dout = torch.empty_like(out)
+        lib, wa, batch = self._lib, self._w_ptr, x.shape[0]
+        # the outputs and their gradient, the partial sums and the scratch in one allocation
+        parts, at = [], 0
+        for count in (lib.rsv_mlp_work_floats(self.num_layers, wa, batch), batch * self.widths[-1],
+                      batch * self.widths[-1], 256, lib.rsv_mlp_scratch_floats(self.num_layers, wa, batch)):
+            parts.append(4 * at)
+            at += (count + 127) // 128 * 128
+        memory = torch.empty(at, dtype=torch.float32, device=self.device)
+        work, out, dout, partials, scratch = (memory.data_ptr() + p for p in parts)
         loss = torch.empty(1, dtype=torch.float32, device=self.device)
-        partials = torch.empty(256, dtype=torch.float32, device=self.device)
-        s = self._stream()
-        check(self._lib.rsv_mlp_mse(out.numel(), out.data_ptr(), target.data_ptr(), dout.data_ptr(),
-                                    loss.data_ptr(), partials.data_ptr(), s))
         grad = torch.empty_like(self.weights)
-        ns = self._lib.rsv_mlp_scratch_floats(self.num_layers, self._w_arr.ctypes.data, x.shape[0])
-        scratch = torch.empty(max(1, ns), dtype=torch.float32, device=self.device)
-        check(self._lib.rsv_mlp_backward(self.num_layers, self._w_arr.ctypes.data, self.weights.data_ptr(),
-                                         x.shape[0], x.data_ptr(), work.data_ptr(), dout.data_ptr(),
-                                         grad.data_ptr(), scratch.data_ptr(), s))
+        s, weights, px = self._stream(), self.weights.data_ptr(), x.data_ptr()
+        check(lib.rsv_mlp_forward(self.num_layers, wa, weights, batch, px, out, work, s))
+        check(lib.rsv_mlp_mse(batch * self.widths[-1], out, target.data_ptr(), dout, loss.data_ptr(), partials, s))
+        check(lib.rsv_mlp_backward(self.num_layers, wa, weights, batch, px, work, dout, grad.data_ptr(), scratch, s))
         return loss, grad
 
     def train(self, x, target, steps: int = 3000, lr: float = 1e-3, beta1: float = 0.9,
@@ -154,7 +154,7 @@ class WarmStartMLP:
         work = self._work(batch)
         out = torch.empty((batch, self.widths[-1]), dtype=torch.float32, device=self.device)
         dout = torch.empty_like(out)
-        ns = self._lib.rsv_mlp_scratch_floats(self.num_layers, self._w_arr.ctypes.data, batch)
+        ns = self._lib.rsv_mlp_scratch_floats(self.num_layers, self._w_ptr, batch)
         scratch = torch.empty(max(1, ns), dtype=torch.float32, device=self.device)
         grad = torch.empty_like(self.weights)
         m = torch.zeros_like(self.weights)
@@ -162,7 +162,7 @@ class WarmStartMLP:
         losses = torch.empty(steps, dtype=torch.float32, device=self.device)
         partials = torch.empty(256, dtype=torch.float32, device=self.device)
         s = self._stream()
-        wa = self._w_arr.ctypes.data
+        wa = self._w_ptr
         lib = self._lib
         for step in range(1, steps + 1):
             check(lib.rsv_mlp_forward(self.num_layers, wa, self.weights.data_ptr(), batch, x.data_ptr(),
