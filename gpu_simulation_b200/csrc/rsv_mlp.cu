@@ -17,9 +17,11 @@
 // flight during a stage, and what follows a product in its epilogue (bias and
 // GELU; GELU's derivative; the bias gradient, which is the row sums of the
 // weight gradient's first operand).  A layer's weight gradient and the gradient
-// of its input are independent and share a launch.  One loss and gradient of the 3-256-256-192
-// network on 512 rows takes 7 launches instead of 15, and 79 us through the Python
-// call against 373 (64 x 64 tiles without prefetch on 16 to 32 CTAs, and column
+// of its input are independent and share a launch.  Where a launch has CTAs to
+// spare a cluster of 2 to 8 shares a tile's depth (a weight gradient's is the
+// number of rows) and adds its parts through distributed shared memory in its order.  One loss
+// and gradient of the 3-256-256-192 network on 512 rows takes 7 launches instead
+// of 15, and 71 us against 373 (64 x 64 tiles without prefetch on 16 to 32 CTAs, and column
 // sums that one thread added over all rows); its error against 64 bits went
 // from 3.4e-7 to 1.0e-7.
 #include <cuda_runtime.h>
@@ -38,6 +40,10 @@ constexpr int kTileK = 16;         // depth of one shared-memory stage
 constexpr int kGroups = 4;         // thread groups sharing the depth
 constexpr int kGroupThreads = 64;  // 8 x 8 threads, 4 x 4 outputs each
 constexpr int kGemmThreads = kGroups * kGroupThreads;
+// CTAs of a launch that shares depths: three a SM.  Loss and gradient on 512 rows,
+// us by this limit: none shared 79, 160 75.7, 296 76.9, 400 to 444 70.7, 592 78.6, 900 85.4; on
+// 32 rows 50 without and 41 with, on 1024 rows 125 and 109.
+constexpr int kMostBlocks = 444;
 constexpr int kPad = kTile + 4;    // 16-byte rows, two-way conflicts at most on the stores
 
 __device__ __forceinline__ float gelu(float z) {
@@ -54,21 +60,27 @@ __device__ __forceinline__ float gelu_grad(float z) {
 struct GemmPair {
   MlpGemm g[2];
   int tiles_n[2], tiles[2];  // column tiles, and all of them
+  int log_splits[2], blocks[2];  // log2 of the CTAs (a cluster) that share a tile's depth; all, in whole clusters
 };
 
+template <bool shared_depth>
 __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constant__ GemmPair P) {
   __shared__ float stage[kGroups][2][2][kTileK][kPad];  // [group][buffer][A, B][k][m or n]
   __shared__ float rows[kGroups][kTile];
-  const int which = static_cast<int>(blockIdx.x) < P.tiles[0] ? 0 : 1;
+  const int which = static_cast<int>(blockIdx.x) < P.blocks[0] ? 0 : 1;
   const MlpGemm &g = P.g[which];
-  const int tile = static_cast<int>(blockIdx.x) - (which ? P.tiles[0] : 0);
+  const int log_splits = shared_depth ? P.log_splits[which] : 0, splits = 1 << log_splits;
+  const int block = static_cast<int>(blockIdx.x) - (which ? P.blocks[0] : 0);
+  const int tile = block >> log_splits, share = block & (splits - 1);
+  if (tile >= P.tiles[which]) return;  // fills up the last cluster
   const int m0 = tile / P.tiles_n[which] * kTile, n0 = tile % P.tiles_n[which] * kTile;
   const int tid = threadIdx.x, group = tid / kGroupThreads, t = tid % kGroupThreads;
   const int tx = t % 8, ty = t / 8;
   const int M = g.M, N = g.N, K = g.K;
   // this group's depth range, whole stages
-  const int span = (K + kGroups * kTileK - 1) / (kGroups * kTileK) * kTileK;
-  const int first = group * span, end = first + span < K ? first + span : K;
+  const int parts = kGroups * splits;
+  const int span = ((K + parts * kTileK - 1) >> (log_splits + 6)) * kTileK;  // 64 = kGroups * kTileK
+  const int first = (share * kGroups + group) * span, end = first + span < K ? first + span : K;
   // threads run along the contiguous index of each operand
   const bool ak = g.sak == 1, bk = g.sbk == 1;
   const int a_m = ak ? t / 16 : t % 32, a_k = ak ? t % 16 : t / 32, a_dm = ak ? 4 : 0, a_dk = ak ? 0 : 2;
@@ -123,21 +135,47 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
     for (int j = 0; j < 4; ++j) part[group * kPart + (4 * ty + i) * kRow + 4 * tx + j] = acc[i][j];
   if (sums) rows[group][t] = row;
   __syncthreads();
-#pragma unroll
-  for (int e = tid; e < kTile * kTile; e += kGemmThreads) {
-    const int i = e / kTile, j = e % kTile, m = m0 + i, n = n0 + j;
-    if (m >= M || n >= N) continue;
-    const float *p = part + i * kRow + j;
-    float z = (p[0] + p[kPart]) + (p[2 * kPart] + p[3 * kPart]);
+  auto finish = [&](int i, int j, float z) {
+    const int m = m0 + i, n = n0 + j;
+    if (m >= M || n >= N) return;
     const long long at = static_cast<long long>(m) * N + n;
     if (g.bias != nullptr) z += g.bias[n];
     if (g.Z != nullptr) g.Z[at] = z;
     if (g.gelu) z = gelu(z);
     if (g.gelu_of != nullptr) z *= gelu_grad(g.gelu_of[at]);
     g.C[at] = z;
+  };
+#pragma unroll
+  for (int e = tid; e < kTile * kTile; e += kGemmThreads) {
+    const int i = e / kTile, j = e % kTile;
+    float *p = part + i * kRow + j;
+    const float z = (p[0] + p[kPart]) + (p[2 * kPart] + p[3 * kPart]);
+    if (!shared_depth || splits == 1) finish(i, j, z);
+    else p[0] = z;  // (only this thread reads the element)
   }
-  if (g.row_sums != nullptr && n0 == 0 && tid < kTile && m0 + tid < M)
-    g.row_sums[m0 + tid] = (rows[0][tid] + rows[1][tid]) + (rows[2][tid] + rows[3][tid]);
+  const bool row_sums = g.row_sums != nullptr && n0 == 0 && tid < kTile;
+  if (row_sums) {
+    const float z = (rows[0][tid] + rows[1][tid]) + (rows[2][tid] + rows[3][tid]);
+    if (shared_depth && splits > 1) rows[0][tid] = z;
+    else if (m0 + tid < M) g.row_sums[m0 + tid] = z;
+  }
+  if (!shared_depth || splits == 1) return;
+  // the cluster's shares, added in its order; each CTA finishes some of the rows
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const int mine = kTile / splits;
+  for (int e = tid; e < mine * kTile; e += kGemmThreads) {
+    const int i = share * mine + e / kTile, j = e % kTile;
+    float z = 0.0f;
+    for (int k = 0; k < splits; ++k) z += *cluster.map_shared_rank(part + i * kRow + j, k);
+    finish(i, j, z);
+  }
+  if (row_sums && share == 0 && m0 + tid < M) {
+    float z = 0.0f;
+    for (int k = 0; k < splits; ++k) z += *cluster.map_shared_rank(&rows[0][tid], k);
+    g.row_sums[m0 + tid] = z;
+  }
+  cluster.sync();  // the shares stay until they are read
 }
 
 // Squared error: dOut = 2 (out - target) / count and the mean, by one cluster
@@ -249,8 +287,32 @@ cudaError_t mlp_gemm(const MlpGemm *g, int count, cudaStream_t s) {
     P.tiles_n[k] = (g[k].N + kTile - 1) / kTile;
     P.tiles[k] = P.tiles_n[k] * ((g[k].M + kTile - 1) / kTile);
   }
-  gemm_kernel<<<P.tiles[0] + P.tiles[1], kGemmThreads, 0, s>>>(P);
-  return cudaGetLastError();
+  // as many CTAs a tile as give every group a stage and keep the launch within kMostBlocks
+  int size = 1;
+  auto plan = [&](int most) {
+    int all = 0;
+    for (int k = 0; k < 2; ++k) {
+      const int splits = P.g[k].K >= most * kGroups * kTileK ? most : 1;
+      P.log_splits[k] = splits == 1 ? 0 : splits == 2 ? 1 : splits == 4 ? 2 : 3;
+      P.blocks[k] = (P.tiles[k] * splits + most - 1) / most * most;
+      all += P.blocks[k];
+    }
+    return all;
+  };
+  for (int most = 2; most <= 8; most *= 2)
+    if (plan(most) <= kMostBlocks && (P.log_splits[0] > 0 || P.log_splits[1] > 0)) size = most;
+  const int blocks = plan(size);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = static_cast<unsigned>(size);
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = size > 1 ? 1 : 0;
+  return size > 1 ? cudaLaunchKernelEx(&cfg, gemm_kernel<true>, P) : cudaLaunchKernelEx(&cfg, gemm_kernel<false>, P);
 }
 
 cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout, float *loss,
