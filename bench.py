@@ -637,7 +637,7 @@ def pass_schedule(n, L):
     from gpu_simulation_b200 import Engine
 
     eng = Engine(n, L, 1.0)
-    eng.set_backward_mode("checkpoint" if n <= 28 else "uncompute")
+    eng.set_backward_mode("checkpoint" if n <= 30 else "uncompute")
     return eng
 
 
