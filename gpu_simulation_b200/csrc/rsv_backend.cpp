@@ -2096,9 +2096,10 @@ void assign_energy_fusion(rsv_backend *B) {
 // 2^n n L for the state.  Up to 4 layers the cluster-resident state is the
 // faster one below 12 qubits (L = 4, energy and gradient: n = 10 18 us against
 // 25, n = 12 37 against 27), and the tile passes never are (n = 12 142 us, n =
-// 28 21 400 against 38).  5 layers cross the cluster at n = 16 (191 us against
-// 180; n = 15 115 against 175).
-bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 16 && L == 5); }
+// 28 21 400 against 38).  5 layers are faster on the ring from 20 qubits on (216
+// us against about 270; n = 16 178 against 125 tiled, n = 17 182 against 146, n = 19
+// 212 against 158; the energy alone 46 against 43, 49 against 57, 53 against 60).
+bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 20 && L == 5); }
 
 // How a single circuit is spread over a cluster (rsv_cluster.cu), the fastest of
 // the measured shapes at L = 8: up to 9 qubits 4 amplitudes a thread on one

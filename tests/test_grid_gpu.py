@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-10
 
 
-@pytest.mark.parametrize("n,layers", [(17, 6), (17, 45), (18, 6), (18, 7), (19, 6), (19, 9), (20, 6), (20, 7), (20, 18),
+@pytest.mark.parametrize("n,layers", [(17, 5), (17, 6), (17, 45), (18, 6), (18, 7), (19, 5), (19, 9), (20, 6), (20, 7), (20, 18),
                                       (20, 30), (20, 64)])
 def test_matches_passes(n, layers):
     import torch

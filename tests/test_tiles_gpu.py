@@ -47,7 +47,7 @@ def test_equal_circuits_in_a_batch(n, layers, count):
         np.testing.assert_allclose(g[off[-2]:], g_ref, atol=TOL, rtol=0)
 
 
-@pytest.mark.parametrize("layers", [6, 7, 20, 64])
+@pytest.mark.parametrize("layers", [5, 6, 7, 20, 64])
 def test_one_circuit_of_16_qubits(layers):
     import torch
 
