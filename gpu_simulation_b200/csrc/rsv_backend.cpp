@@ -2414,7 +2414,9 @@ rsv_status rsv_create(int num_qubits, int num_layers, double field, const char *
     }
     // energy partials before the plan: a fused energy adds a pass's share
     B->energy_grid = energy_grid_size(num_qubits, B->sms);
-    B->energy_partials.alloc(static_cast<size_t>(B->energy_grid) + 4 * static_cast<size_t>(std::max(1, B->sms)));
+    // (and the ring contraction keeps a value a chain there, whatever the device has)
+    B->energy_partials.alloc(std::max(static_cast<size_t>(B->energy_grid) + 4 * static_cast<size_t>(std::max(1, B->sms)),
+                                      static_cast<size_t>(kRingMaxParts)));
     setup_plan(B.get(), RSV_BACKWARD_AUTO);
     const size_t nl = static_cast<size_t>(num_qubits) * num_layers;
     if (strat == "dense_scan") {

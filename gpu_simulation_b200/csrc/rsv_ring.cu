@@ -60,7 +60,8 @@ namespace {
 constexpr int kComps = 5;  // I, X, H, W, S
 constexpr int kI = 0, kX = 1, kH = 2, kW = 3, kS = 4;
 constexpr int kSweepThreads = 32 * (kComps + 1);
-constexpr int kGradWarps = 2 * kComps;
+constexpr int kGradWarps = kRingGradWarps;
+static_assert(kGradWarps == 2 * kComps, "two warps a component");
 constexpr int kMaxDerivs = kRingDerivs;
 
 struct SiteM {  // cos, sin of the full angles of a wire's last layer
@@ -489,7 +490,7 @@ __device__ __forceinline__ Mat<R, DB> load_rows(const double2 *p, bool mirror, i
 // Chains of one step of ring_grad_kernel: 256 elements of each matrix kind.
 template <int DB>
 __host__ __device__ constexpr int chains_a_step() {
-  return DB == 1 ? 4 : 1;
+  return ring_chains_a_step(DB == 1 ? 4 : 5);
 }
 
 __device__ __forceinline__ void copy16(double2 *to, const double2 *from) {
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(32 * kGradWarps, 1) ring_grad_kernel(const Rin
   const int worker = rank * kGradWarps + warp, workers = G_ctas * kGradWarps;
   if (w == 0) {
     // T_0's column a from the pairs (a, .): sum over the bra bits and over ab
-    const int share = workers / bond;  // warps a column
+    const int share = workers / bond;  // warps a column (one at least: ring_gradient_ctas)
     if (worker < share * bond) {
       const int a = worker % bond;
       double gr[DB], gi[DB];
@@ -797,14 +798,10 @@ cudaError_t gradient(const RingParams &P, cudaStream_t s) {
   constexpr size_t smem = sizeof(double2) * (2 + kGradWarps / DB + 8 * chains_a_step<DB>() * kComps) * 64 * DB * DB;
   cudaError_t e = set_smem_limit_once(ring_grad_kernel<DB>, smem, done);
   if (e != cudaSuccess) return e;
-  // at most eight CTAs a site, no more than its chains need, and no more (one CTA
-  // an SM) than fill the SMs once
-  const int steps = (ring_chains(P.L) + chains_a_step<DB>() - 1) / chains_a_step<DB>();
-  int ctas = steps < 8 ? steps : 8;
   int dev = 0, sms = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  while (ctas > 1 && ctas * P.n > sms) --ctas;
+  const int ctas = ring_gradient_ctas(P.n, P.L, sms);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(P.n));
   cfg.blockDim = dim3(32 * kGradWarps);
