@@ -1362,7 +1362,8 @@ void run_gate_level(rsv_backend *B, bool grad, double *energy_out, double *grad_
 }
 
 // d_params: the angles on the device, or null when B->coef holds their cosines
-// and sines.  keep: an energy-only call whose gradient may be asked for later.
+// and sines.  keep: an energy-only call whose gradient may be asked for later
+// (rsv_backward_device).
 void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_out, double *grad_out,
              cudaStream_t st, bool keep = false) {
   ++B->generation;
@@ -1376,11 +1377,12 @@ void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_o
       check(launch_coef(d_params, B->coef.p, static_cast<int>(B->n * B->L), st), "coef launch");
     });
   }
-  if (B->gate_level) {
+  // (the split entry points run the tile passes, whose state the backward takes up)
+  if (B->gate_level && !keep) {
     run_gate_level(B, grad, energy_out, grad_out, st);
     return;
   }
-  if (B->dense) {
+  if (B->dense && !keep) {
     DenseArgs D{};
     D.n = B->n;
     D.L = B->L;
@@ -2417,8 +2419,8 @@ rsv_status rsv_create(int num_qubits, int num_layers, double field, const char *
     // (and the ring contraction keeps a value a chain there, whatever the device has)
     B->energy_partials.alloc(std::max(static_cast<size_t>(B->energy_grid) + 4 * static_cast<size_t>(std::max(1, B->sms)),
                                       static_cast<size_t>(kRingMaxParts)));
-    setup_plan(B.get(), RSV_BACKWARD_AUTO);
     const size_t nl = static_cast<size_t>(num_qubits) * num_layers;
+    // the strategy before the plan: choose_path leaves the other two their own kernels
     if (strat == "dense_scan") {
       B->dense = true;
       B->dense_work.alloc(dense_workspace_bytes(num_qubits, num_layers) / sizeof(double2));
@@ -2428,6 +2430,7 @@ rsv_status rsv_create(int num_qubits, int num_layers, double field, const char *
       B->gate_grid = gate_grid(num_qubits, B->sms);
       B->gate_partials.alloc(static_cast<size_t>(B->gate_grid) * (1 + 2 * nl));
     }
+    setup_plan(B.get(), RSV_BACKWARD_AUTO);
     B->coef.alloc(nl);
     B->ptab.alloc(static_cast<size_t>(num_layers) * 1024);
     B->outputs.alloc(1 + B->num_params);
@@ -2821,6 +2824,8 @@ rsv_status rsv_describe_backend(rsv_backend *B, char *buf, size_t buf_size, size
     os << "analytic_layers=" << B->analytic_layers << " kernels=" << B->kernel_flags
        << " high_tile_c=" << (B->force_c ? std::to_string(B->force_c) : std::string("planner"))
        << " tma_passes=" << B->tma_passes;
+    if (B->gate_level) os << " gate_level (the plan below is not used, but by the split entry points)";
+    if (B->dense) os << " dense_scan (the plan below is not used, but by the split entry points)";
     if (B->path == Path::kRing) os << " ring_contraction (the plan below is not used)";
     if (B->path == Path::kCluster)
       os << (B->n > kClusterMaxQubits ? " whole_device: a CTA a SM"

@@ -69,9 +69,10 @@ const char *rsv_stage_name(int i);
  * "inverse_walk_cuQuantum" (alias "inverse_walk_cuquantum": RY, RZ and CNOT as
  * separate kernels and the gate-level adjoint walk, without cuStateVec) or
  * "dense_scan" (n <= 8: dense layer matrices, product tree on FP64 tensor
- * cores); results agree to rounding.  The split device entry points
- * (rsv_forward_device / rsv_backward_device) and rsv_benchmark_forward_graph
- * always run the tile-pass engine.  structured_rotation_chunk_width must be in
+ * cores); results agree to rounding.  Engines of the last two run the split
+ * device entry points (rsv_forward_device / rsv_backward_device) on the tile
+ * passes, and rsv_benchmark_forward_graph times the tile passes' forward for
+ * every engine.  structured_rotation_chunk_width must be in
  * [1, 8] and double_buffer is accepted; both are validated as the reference
  * does and otherwise ignored (the engine plans its own tiles).
  * Allocates three state buffers of 16 * 2^max(n,12) bytes.
