@@ -1568,6 +1568,11 @@ struct rsv_batch {
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> joined;
   cudaEvent_t forked = nullptr;
+  // Runs read the descriptors and vectors above on the callers' streams:
+  // `done` is behind the last of them; `untracked` says that there may be others
+  // (replays of a captured run, or the launches of one that failed half-way).
+  cudaEvent_t done = nullptr;
+  bool untracked = false;
 };
 
 namespace rsv {
@@ -1603,6 +1608,12 @@ int batch_plan_index(rsv_batch *Bt, int n, int L) {
   Bt->plan_cost.push_back(cost);
   Bt->dirty = true;
   return static_cast<int>(Bt->plans.size()) - 1;
+}
+
+// Waits for the runs enqueued so far, before what they read is rewritten or freed.
+void batch_wait(rsv_batch *Bt) {
+  if (Bt->untracked) check(cudaDeviceSynchronize(), "batch wait");
+  else if (Bt->done != nullptr) check(cudaEventSynchronize(Bt->done), "batch wait");
 }
 
 template <typename T>
@@ -1814,6 +1825,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
         Bt->plan_cost[static_cast<size_t>(C.plan)] * static_cast<double>(u64{1} << std::max(n, kTileBits));
     off += static_cast<size_t>(2) * n * L;
   }
+  batch_wait(Bt);
   if (Bt->resident && count > 0 && !batch_classes(Bt, circ)) Bt->resident = false;
   cudaStream_t st = Bt->stream;
   if (Bt->dirty) {
@@ -1831,10 +1843,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
   batch_group(Bt);
 }
 
-void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad,
-               cudaStream_t st) {
-  if (Bt->count == 0) return;
-  if (d_params == nullptr || d_energy == nullptr) invalid("null device pointer");
+void batch_launch(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad, cudaStream_t st) {
   if (Bt->resident) {
     auto launch = [&](const rsv_batch::Class &c, cudaStream_t s) {
       ClusterArgs A{};
@@ -1889,6 +1898,22 @@ void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *
   if (grid > Bt->slots) invalid("fewer scratch slots than one thread-block cluster");
   check(cudaMemsetAsync(Bt->d_counter.p, 0, sizeof(int), st), "batch counter reset");
   check(launch_batch(A, grid, C, st), "batch launch");
+}
+
+void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad,
+               cudaStream_t st) {
+  if (Bt->count == 0) return;
+  if (d_params == nullptr || d_energy == nullptr) invalid("null device pointer");
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
+  if (Bt->done == nullptr)
+    check(cudaEventCreateWithFlags(&Bt->done, cudaEventDisableTiming), "cudaEventCreate");
+  const bool untracked = Bt->untracked;
+  Bt->untracked = true;
+  batch_launch(Bt, d_params, d_energy, d_grad, st);
+  if (capture != cudaStreamCaptureStatusNone) return;  // its replays are known to the caller alone
+  check(cudaEventRecord(Bt->done, st), "cudaEventRecord");
+  Bt->untracked = untracked;
 }
 
 }  // namespace
@@ -2935,6 +2960,10 @@ rsv_status rsv_batch_destroy(rsv_batch *batch) {
     if (batch == nullptr) return;
     cudaStreamSynchronize(batch->stream);
     cudaStreamDestroy(batch->stream);
+    if (batch->done) {
+      cudaEventSynchronize(batch->done);
+      cudaEventDestroy(batch->done);
+    }
     for (auto s : batch->side) cudaStreamDestroy(s);
     for (auto e : batch->joined) cudaEventDestroy(e);
     if (batch->forked) cudaEventDestroy(batch->forked);
@@ -2980,7 +3009,7 @@ rsv_status rsv_batch_set_cluster(rsv_batch *batch, int cluster) {
     if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) invalid("cluster must be 1, 2, 4 or 8");
     if (cluster > batch->slots) invalid("cluster exceeds the scratch slots");
     if (batch_max_active_clusters(cluster) < 1) invalid("no cluster of this size fits on the device");
-    check(cudaStreamSynchronize(batch->stream), "batch synchronize");
+    batch_wait(batch);
     batch->cluster = cluster;
     batch->resident = false;
     batch_group(batch);
@@ -2991,6 +3020,7 @@ rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident) {
   return guarded([&] {
     const OnDevice on_device(batch ? batch->device : -1);
     if (batch == nullptr) invalid("batch is null");
+    if (resident) batch_wait(batch);
     batch->resident = resident != 0;
     if (batch->resident && batch->count > 0 && !batch_classes(batch, batch->circuits)) {
       batch->resident = false;

@@ -349,7 +349,10 @@ unsigned long long rsv_ring_map(unsigned long long index, int num_qubits, int in
  *
  * rsv_batch_set_circuits builds (or reuses) the pass plan of every distinct
  * (num_qubits, num_layers), sorts the circuits by decreasing cost and uploads
- * the descriptors; it is synchronous.  rsv_batch_run_device enqueues the
+ * the descriptors; it is synchronous and waits for the runs enqueued before,
+ * which read them (rsv_batch_set_resident and rsv_batch_set_cluster do too).
+ * A graph that captured a run is void after any of the three.
+ * rsv_batch_run_device enqueues the
  * whole batch on `stream` (used as given; 0 = legacy default stream), with
  * the launches of further qubit counts on streams forked from it and joined to
  * it again: no allocation and no host synchronisation, so it can be captured
