@@ -1553,7 +1553,8 @@ struct rsv_batch {
   cudaStream_t stream = nullptr;
   // Cluster-resident circuits (rsv_cluster.cu), the default: one launch per
   // qubit count, largest first, on streams forked from the caller's.  A caller
-  // that gave slots, or set them or a cluster size, chose the persistent kernel.
+  // that gave slots, or set them or a cluster size, chose the persistent kernel;
+  // circuits whose clusters or vectors do not fit take it too (`classes` empty).
   bool resident = true;
   struct Class {
     int n, first, count, max_layers, clusters;
@@ -1826,7 +1827,8 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
     off += static_cast<size_t>(2) * n * L;
   }
   batch_wait(Bt);
-  if (Bt->resident && count > 0 && !batch_classes(Bt, circ)) Bt->resident = false;
+  Bt->classes.clear();
+  if (Bt->resident && count > 0 && !batch_classes(Bt, circ)) Bt->classes.clear();
   cudaStream_t st = Bt->stream;
   if (Bt->dirty) {
     upload(Bt->d_plans, Bt->plans, st, "batch plan upload");
@@ -1844,7 +1846,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
 }
 
 void batch_launch(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad, cudaStream_t st) {
-  if (Bt->resident) {
+  if (!Bt->classes.empty()) {
     auto launch = [&](const rsv_batch::Class &c, cudaStream_t s) {
       ClusterArgs A{};
       A.n = c.n;
@@ -2999,6 +3001,7 @@ rsv_status rsv_batch_set_active_slots(rsv_batch *batch, int slots) {
       invalid("slots must be in [1, " + std::to_string(batch->slots) + "]");
     batch->active_slots = slots;
     batch->resident = false;
+    batch->classes.clear();
   });
 }
 
@@ -3012,6 +3015,7 @@ rsv_status rsv_batch_set_cluster(rsv_batch *batch, int cluster) {
     batch_wait(batch);
     batch->cluster = cluster;
     batch->resident = false;
+    batch->classes.clear();
     batch_group(batch);
   });
 }
@@ -3022,8 +3026,10 @@ rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident) {
     if (batch == nullptr) invalid("batch is null");
     if (resident) batch_wait(batch);
     batch->resident = resident != 0;
+    batch->classes.clear();
     if (batch->resident && batch->count > 0 && !batch_classes(batch, batch->circuits)) {
       batch->resident = false;
+      batch->classes.clear();
       throw Error(RSV_ERR_UNSUPPORTED, "a cluster of these circuits does not fit the device");
     }
   });

@@ -377,7 +377,8 @@ rsv_status rsv_batch_info(rsv_batch *batch, int *count, size_t *num_params, int 
                           size_t *device_bytes);
 
 /* Run the following batches cluster-resident (non-zero) or on the persistent
- * kernel. */
+ * kernel.  A later list whose circuits' memory cannot be had resident takes the
+ * persistent kernel for itself alone. */
 rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident);
 
 /* CTAs in flight for the following runs (1..the slots given at creation;

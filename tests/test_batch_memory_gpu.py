@@ -1,0 +1,55 @@
+"""Batches on a device that is almost full."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpu_simulation_b200 import BatchEngine
+from gpu_simulation_b200.batch import param_offsets
+
+pytestmark = pytest.mark.gpu
+
+
+def fill_device(leave: int):
+    """All of the device's free memory but `leave` bytes."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+
+
+def circuits(ns, ls, seed):
+    rng = np.random.default_rng(seed)
+    return rng.uniform(0.2, 2.0, len(ns)), rng.uniform(0.0, 2.0 * np.pi, int(param_offsets(ns, ls)[-1]))
+
+
+def test_one_list_without_room_does_not_change_the_next_ones():
+    import torch
+
+    ns, ls = [16] * 160, [1, 2, 3, 4, 5] * 32  # 4 vectors of 1 MiB for each circuit in flight: 144 MiB on clusters of 4
+    hs, p = circuits(ns, ls, 1)
+    small = ([13, 12, 9, 6], [5, 4, 3, 7])
+    hs_small, p_small = circuits(*small, 2)
+    fresh = BatchEngine()
+    e_ref, g_ref = fresh.energy_and_grad(ns, ls, hs, p)
+    e_small, g_small = fresh.energy_and_grad(*small, hs_small, p_small)
+    fresh.set_cluster(8)
+    e_pers, g_pers = fresh.energy_and_grad(*small, hs_small, p_small)
+    assert not np.array_equal(g_small, g_pers)  # the two kernels are told apart by their last bits
+    fresh.close()
+    eng = BatchEngine()
+    full = fill_device(32 << 20)
+    e, g = eng.energy_and_grad(ns, ls, hs, p)
+    del full
+    torch.cuda.empty_cache()
+    np.testing.assert_allclose(e, e_ref, atol=1e-10, rtol=0)
+    np.testing.assert_allclose(g, g_ref, atol=1e-10, rtol=0)
+    assert not np.array_equal(g, g_ref)  # it did take the other kernel
+    e, g = eng.energy_and_grad(*small, hs_small, p_small)
+    assert np.array_equal(e, e_small) and np.array_equal(g, g_small)
+    e, g = eng.energy_and_grad(ns, ls, hs, p)
+    assert np.array_equal(e, e_ref) and np.array_equal(g, g_ref)
+    eng.close()
