@@ -814,7 +814,12 @@ struct DevBuf {
   void alloc(size_t n) {
     release();
     if (n == 0) return;
-    check(cudaMalloc(&p, n * sizeof(T)), "cudaMalloc");
+    const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();  // reported by the exception; other code's next check must not find it
+    }
+    check(e, "cudaMalloc");
     count = n;
     owned = true;
   }

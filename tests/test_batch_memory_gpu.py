@@ -53,3 +53,17 @@ def test_one_list_without_room_does_not_change_the_next_ones():
     e, g = eng.energy_and_grad(ns, ls, hs, p)
     assert np.array_equal(e, e_ref) and np.array_equal(g, g_ref)
     eng.close()
+
+
+def test_a_refused_allocation_is_not_left_for_others_to_find():
+    import torch
+
+    eng = BatchEngine()
+    many = 4_000_000  # descriptors of 32 and about 40 bytes, allocated half as large again
+    full = fill_device(256 << 20)
+    with pytest.raises((MemoryError, RuntimeError)):
+        eng.set_circuits(np.full(many, 2), np.ones(many), np.ones(many))
+    assert int(full[:4].fill_(3).sum()) == 12  # torch checks the last error at its launches
+    del full
+    torch.cuda.empty_cache()
+    eng.close()
