@@ -1543,7 +1543,9 @@ struct rsv_batch {
   rsv::DevBuf<rsv::BatchStep> d_steps;
   rsv::DevBuf<rsv::BatchTile> d_tiles;
   rsv::DevBuf<int> d_undo;
-  // current circuits
+  // current circuits; `whole`: all of what describes them is up to date (false
+  // where a description failed half-way)
+  bool whole = true;
   int count = 0;
   size_t num_params = 0;
   std::vector<rsv::BatchCircuit> circuits;
@@ -1614,6 +1616,10 @@ int batch_plan_index(rsv_batch *Bt, int n, int L) {
   Bt->plan_cost.push_back(cost);
   Bt->dirty = true;
   return static_cast<int>(Bt->plans.size()) - 1;
+}
+
+void batch_check_whole(const rsv_batch *Bt) {
+  if (!Bt->whole) invalid("the batch's circuits could not be set up; describe them again");
 }
 
 // Waits for the runs enqueued so far, before what they read is rewritten or freed.
@@ -1832,6 +1838,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
     off += static_cast<size_t>(2) * n * L;
   }
   batch_wait(Bt);
+  Bt->whole = false;
   Bt->classes.clear();
   if (Bt->resident && count > 0 && !batch_classes(Bt, circ)) Bt->classes.clear();
   cudaStream_t st = Bt->stream;
@@ -1848,6 +1855,7 @@ void batch_set_circuits(rsv_batch *Bt, int count, const int *ns, const int *Ls, 
   Bt->count = count;
   Bt->num_params = off;
   batch_group(Bt);
+  Bt->whole = true;
 }
 
 void batch_launch(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad, cudaStream_t st) {
@@ -1909,6 +1917,7 @@ void batch_launch(rsv_batch *Bt, const double *d_params, double *d_energy, doubl
 
 void batch_run(rsv_batch *Bt, const double *d_params, double *d_energy, double *d_grad,
                cudaStream_t st) {
+  batch_check_whole(Bt);
   if (Bt->count == 0) return;
   if (d_params == nullptr || d_energy == nullptr) invalid("null device pointer");
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -3017,11 +3026,14 @@ rsv_status rsv_batch_set_cluster(rsv_batch *batch, int cluster) {
     if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) invalid("cluster must be 1, 2, 4 or 8");
     if (cluster > batch->slots) invalid("cluster exceeds the scratch slots");
     if (batch_max_active_clusters(cluster) < 1) invalid("no cluster of this size fits on the device");
+    batch_check_whole(batch);
     batch_wait(batch);
     batch->cluster = cluster;
     batch->resident = false;
     batch->classes.clear();
+    batch->whole = false;
     batch_group(batch);
+    batch->whole = true;
   });
 }
 
@@ -3029,14 +3041,18 @@ rsv_status rsv_batch_set_resident(rsv_batch *batch, int resident) {
   return guarded([&] {
     const OnDevice on_device(batch ? batch->device : -1);
     if (batch == nullptr) invalid("batch is null");
+    batch_check_whole(batch);
     if (resident) batch_wait(batch);
     batch->resident = resident != 0;
     batch->classes.clear();
+    batch->whole = !batch->resident;
     if (batch->resident && batch->count > 0 && !batch_classes(batch, batch->circuits)) {
       batch->resident = false;
       batch->classes.clear();
+      batch->whole = true;  // (the persistent kernel's description stands)
       throw Error(RSV_ERR_UNSUPPORTED, "a cluster of these circuits does not fit the device");
     }
+    batch->whole = true;
   });
 }
 

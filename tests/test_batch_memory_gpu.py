@@ -67,3 +67,34 @@ def test_a_refused_allocation_is_not_left_for_others_to_find():
     del full
     torch.cuda.empty_cache()
     eng.close()
+
+
+def test_a_description_that_failed_is_not_run():
+    import torch
+
+    ns, ls = [12, 9], [3, 4]
+    hs, p = circuits(ns, ls, 3)
+    eng = BatchEngine()
+    e_ref, g_ref = eng.energy_and_grad(ns, ls, hs, p)
+    d = torch.tensor(p, device="cuda")
+    e, g = torch.zeros(2, dtype=torch.float64, device="cuda"), torch.zeros_like(d)
+    many = 4_000_000
+    full = fill_device(256 << 20)
+    with pytest.raises((MemoryError, RuntimeError)):
+        eng.set_circuits(np.full(many, 2), np.ones(many), np.ones(many))
+    with pytest.raises(ValueError):
+        eng.run_device(d, e, g)
+    with pytest.raises(ValueError):
+        eng.set_cluster(1)
+    with pytest.raises(ValueError):
+        eng.set_resident(True)
+    del full
+    torch.cuda.empty_cache()
+    assert not g.any()
+    e2, g2 = eng.energy_and_grad(ns, ls, hs, p)
+    assert np.array_equal(e2, e_ref) and np.array_equal(g2, g_ref)
+    with pytest.raises(ValueError):  # refused before anything is touched: the list before stands
+        eng.set_circuits([12, 17], [1, 1], [1.0, 1.0])
+    eng.run_device(d, e, g)
+    assert np.array_equal(g.cpu().numpy(), g_ref)
+    eng.close()
