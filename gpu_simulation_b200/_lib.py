@@ -52,6 +52,7 @@ _SIGNATURES = {
     "rsv_set_backward_mode": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rsv_set_analytic_layers": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rsv_set_kernels": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
+    "rsv_set_barrier_polls": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rsv_batch_set_cluster": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rsv_batch_set_resident": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rsv_batch_cluster": ([ctypes.c_void_p, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),

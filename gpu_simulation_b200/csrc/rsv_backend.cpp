@@ -915,6 +915,7 @@ struct rsv_backend {
   // field of the last forward
   rsv::Path path = rsv::Path::kPasses;
   rsv::ClusterShape cluster_shape{0, 4, true};
+  int barrier_polls = rsv::kGridPolls;  // rsv_set_barrier_polls
   double forward_field = 0.0;
   rsv::DevBuf<int> tables;  // pass_grid | theta_pass | theta_slot | phi_pass
   rsv::DevBuf<int> order;   // undo order of the wires within a backward layer
@@ -1292,7 +1293,7 @@ ClusterArgs cluster_args(rsv_backend *B, const double *d_params, double *energy_
   A.n = B->n;
   A.shape = B->cluster_shape;
   A.memory = B->states.p;
-  if (B->n > kClusterMaxQubits) A.counter = B->pipeline_err.p;
+  A.polls = B->barrier_polls;
   A.count = 1;
   A.item.L = A.max_layers = B->L;
   A.item.h = B->forward_field;
@@ -1409,15 +1410,21 @@ void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_o
   run_finalize(B, grad, energy_out, grad_out, st, fused, store);
 }
 
-// After a synchronised call: a NaN energy from a backend with TMA passes may
-// come from a pipeline wait that gave up (finalize_kernel writes NaN then);
-// report it as an error and clear the flag.
-void check_pipeline(rsv_backend *B, double energy) {
-  if ((B->tma_passes == 0 && B->path != Path::kCluster) || !std::isnan(energy)) return;
+// After a synchronised call: a NaN energy may come from a wait that gave up, of
+// a TMA pass for its pipeline (finalize_kernel writes NaN then; the flag is
+// cleared) or of a whole-device kernel for its other blocks (its next call clears
+// the flag).  Report it as an error.  `outputs`: energy, then the gradient if any.
+void check_pipeline(rsv_backend *B, const double *outputs, bool grad) {
+  if (!std::isnan(outputs[0]) && !(grad && std::isnan(outputs[1]))) return;
   int flag = 0;
-  check(cudaMemcpy(&flag, B->pipeline_err.p, sizeof(int), cudaMemcpyDeviceToHost), "pipeline flag read");
+  if (B->path == Path::kPasses && B->tma_passes > 0) {
+    check(cudaMemcpy(&flag, B->pipeline_err.p, sizeof(int), cudaMemcpyDeviceToHost), "pipeline flag read");
+    if (flag != 0) check(cudaMemset(B->pipeline_err.p, 0, sizeof(int)), "pipeline flag clear");
+  } else if (B->path == Path::kCluster && B->n > kClusterMaxQubits) {
+    check(cudaMemcpy(&flag, grid_lost_flag(cluster_args(B, nullptr, nullptr, nullptr)), sizeof(int), cudaMemcpyDeviceToHost),
+          "barrier flag read");
+  }
   if (flag == 0) return;
-  check(cudaMemset(B->pipeline_err.p, 0, sizeof(int)), "pipeline flag clear");
   throw Error(RSV_ERR_CUDA, "a kernel gave up waiting for its pipeline or its other blocks (flag " +
                                 std::to_string(flag) + "); the results of this call are void");
 }
@@ -2522,7 +2529,7 @@ rsv_status rsv_energy_and_grad(rsv_backend *B, const double *params, size_t num_
             "result download");
     }
     check(cudaStreamSynchronize(st), "energy_and_grad");
-    check_pipeline(B, B->out_host.p[0]);
+    check_pipeline(B, B->out_host.p, grad);
     *energy_out = B->out_host.p[0];
     if (grad) std::memcpy(gradient_out, B->out_host.p + 1, B->num_params * sizeof(double));
   });
@@ -2652,6 +2659,7 @@ rsv_status rsv_profile_energy_and_grad(rsv_backend *B, const double *params, siz
     cudaEventElapsedTime(&ms, ev[4], ev[5]);
     stage_ms_out[7] = ms;
     for (auto &e : ev) cudaEventDestroy(e);
+    check_pipeline(B, B->out_host.p, grad);
     *energy_out = B->out_host.p[0];
     if (grad) std::memcpy(gradient_out, B->out_host.p + 1, B->num_params * sizeof(double));
   });
@@ -2771,6 +2779,14 @@ rsv_status rsv_set_kernels(rsv_backend *B, int flags) {
     check(cudaStreamSynchronize(B->stream), "backend synchronize");
     B->kernel_flags = flags;
     setup_plan(B, B->backward_mode);
+  });
+}
+
+rsv_status rsv_set_barrier_polls(rsv_backend *B, int polls) {
+  return guarded([&] {
+    if (B == nullptr) invalid("backend is null");
+    if (polls < 0) invalid("polls must not be negative");
+    B->barrier_polls = polls;
   });
 }
 

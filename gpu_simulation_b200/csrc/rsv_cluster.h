@@ -32,8 +32,7 @@ struct ClusterArgs {
   ClusterShape shape;
   int count;                   // circuits
   int clusters;                // with a counter (tiled): clusters that take them in turn
-  int *counter;                // 0 at the launch, or null: one cluster a circuit; whole device: set where a
-                               // CTA gave up waiting for the others
+  int *counter;                // 0 at the launch, or null: one cluster a circuit
   double2 *memory;             // clusters * cluster_memory_values(n, shape, max_layers)
   const ClusterItem *items;    // [count], or null: the one circuit `item`
   ClusterItem item;
@@ -48,7 +47,11 @@ struct ClusterArgs {
   // checkpoints) and runs the backward alone.
   double2 *psi, *lam;
   int resume;
+  int polls;                   // whole device: how often a CTA polls a barrier before it gives up
 };
+
+// Polls of a whole-device barrier: about a second.
+constexpr int kGridPolls = 1 << 21;
 
 bool cluster_shape_built(int n, ClusterShape h);
 // Global memory of a cluster: psi's checkpoints, or a tiled circuit's vectors.
@@ -68,5 +71,7 @@ constexpr int kGridMaxQubits = 20;
 size_t grid_memory_values(int n, int max_layers);
 cudaError_t launch_grid(const ClusterArgs &A, cudaStream_t s);
 cudaError_t grid_capacity(int n, int max_layers, int *circuits);
+// On the device: non-zero where the circuit's last call gave up; all of its results are NaN.
+const unsigned *grid_lost_flag(const ClusterArgs &A);
 
 }  // namespace rsv

@@ -40,37 +40,51 @@ constexpr int kMostGridCtas = 256;
 // values of register bits, total, lane bits, tile bits, warp bits; theta sums of 0..11
 constexpr int kGridRec = 48, kGridHigh = 4, kGridPhi = 8, kGridTotal = 12, kGridLane = 13, kGridTile = 18, kGridWarp = 26,
               kGridLow = 32;
-// How often a CTA looks whether the others have arrived (about a second), then
-// it gives up for all of them.
-constexpr int kGridSpins = 1 << 21;
-constexpr int kGridLost = 1 << 8;  // what the caller's flag then holds
-
 // Behind the four vectors: records [layer][value][CTA], energies [CTA], then
 struct GridState {
-  unsigned arrived, failed;  // 0 at the launch
+  unsigned arrived;  // CTAs that came to a barrier, all barriers; 0 at the launch
+  unsigned lost;     // set by a launch that gave up; 0 at a call's first launch
 };
+constexpr unsigned kGridVoid = 1u << 31;  // of `arrived`: a CTA gave up waiting
 
 // Barrier of the grid: what its CTAs stored is there for loads that go to L2.
-// False, at every CTA sooner or later, where one did not arrive.
-__device__ __forceinline__ bool sync_grid(GridState *S, unsigned &target) {
+// A CTA looks `polls` times whether the others have arrived, then it gives up for
+// all of them.  It does so in the word that counts them, and only while that is
+// still short: so either no CTA passes a barrier or every one does, and none is
+// left with results that the others void.
+__device__ __forceinline__ bool sync_grid(GridState *S, unsigned &target, int polls) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     target += gridDim.x;
     __threadfence();
-    atomicAdd(&S->arrived, 1u);
-    int spins = 0;
-    unsigned seen, failed;
-    do {
+    unsigned seen = atomicAdd(&S->arrived, 1u) + 1;
+    // (a void word is above every target)
+#pragma unroll 1
+    for (int k = 0; seen < target && k < polls; ++k) {
+      // (the second load spaces the polls out: n = 20, L = 8 418 us against 434 without it, n = 17 166 at
+      // L = 6 against 171)
+      unsigned spare;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&S->arrived) : "memory");
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(failed) : "l"(&S->failed) : "memory");
-    } while (seen < target && !failed && ++spins < kGridSpins);
-    if (seen < target) atomicExch(&S->failed, 1u);
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(spare) : "l"(&S->lost) : "memory");
+    }
+#pragma unroll 1
+    while (seen < target) {  // (no more turns than CTAs: each one that fails found another arrival)
+      const unsigned was = atomicCAS(&S->arrived, seen, seen | kGridVoid);
+      seen = was == seen ? seen | kGridVoid : was;
+    }
     __threadfence();
-    ok = seen >= target;
+    ok = seen < kGridVoid;
   }
   __syncthreads();
   return ok != 0;
+}
+
+__host__ __device__ inline size_t grid_doubles(int max_layers) {  // behind the vectors, without the state
+  return static_cast<size_t>(max_layers) * kGridRec * kMostGridCtas + kMostGridCtas;
+}
+__host__ __device__ inline GridState *grid_state(const ClusterArgs &A, int n) {
+  return reinterpret_cast<GridState *>(reinterpret_cast<double *>(A.memory + (size_t{4} << n)) + grid_doubles(A.max_layers));
 }
 
 template <int n>
@@ -85,7 +99,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
   unsigned char *bufP = smem, *bufL = smem + kGridBuf;
   double *recs = reinterpret_cast<double *>(A.memory + (size_t{4} << n));
   double *energies = recs + static_cast<size_t>(A.max_layers) * kGridRec * kMostGridCtas;
-  GridState *S = reinterpret_cast<GridState *>(energies + kMostGridCtas);
+  GridState *S = grid_state(A, n);
   unsigned arrivals = 0;
   const Tables T = build_tables<G>(A.params ? A.params + item.param_off : nullptr, A.coef, cta == 0 ? A.coef_out : nullptr,
                                    L, smem, 2 * kGridBuf);
@@ -143,7 +157,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
       const unsigned flip = T.flip[l];
       const double *rot = T.rot + l * n;
       double2 a[16];
-      if (!sync_grid(S, arrivals)) return false;
+      if (!sync_grid(S, arrivals, A.polls)) return false;
       for (unsigned tile = cta; tile < G::tiles; tile += ctas) {
 #pragma unroll
         for (int r = 0; r < 16; ++r) a[r] = __ldcg(psi0 + (tile << 12 | u_b | r << 4));
@@ -164,7 +178,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
         for (int r = 0; r < 16; ++r) psi0[tile << 12 | u_a | (static_cast<unsigned>(r) ^ x) << 8] = a[r];
         __syncthreads();  // the buffer is read
       }
-      if (!sync_grid(S, arrivals)) return false;
+      if (!sync_grid(S, arrivals, A.polls)) return false;
       const double2 *tab = T.phase + static_cast<size_t>(l) * nt * 16;
       const double scale = T.scale[l];
       for (unsigned tile = cta; tile < G::tiles; tile += ctas) {
@@ -189,7 +203,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
       }
       swap(psi0, psi1);
     }
-    if (!sync_grid(S, arrivals)) return false;
+    if (!sync_grid(S, arrivals, A.polls)) return false;
     // ---- lambda = H psi and the energy, on low tiles
     const bool keep = A.grad_out != nullptr || A.lam != nullptr;
     double energy = 0.0;
@@ -243,7 +257,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
       for (int k = 0; k < G::warps; ++k) s += T.red[k];
       energies[cta] = s;
     }
-    if (!sync_grid(S, arrivals)) return false;  // the energies and H psi are there
+    if (!sync_grid(S, arrivals, A.polls)) return false;  // the energies and H psi are there
     if (cta == 0 && warp == 0 && A.energy_out != nullptr) {
       double s = 0.0;
       for (unsigned k = lane; k < ctas; k += 32) s += __ldcg(energies + k);
@@ -346,7 +360,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
     }
     swap(psi0, psi1);
     swap(lam0, lam1);
-    if (!sync_grid(S, arrivals)) return false;
+    if (!sync_grid(S, arrivals, A.polls)) return false;
     {  // low pass, in place
       double theta[12];
 #pragma unroll
@@ -408,7 +422,7 @@ __device__ __forceinline__ bool run_grid(const ClusterArgs &A, unsigned char *sm
         rec[static_cast<size_t>(kGridLow + lane) * ctas] = s;
       }
     }
-    if (!sync_grid(S, arrivals)) return false;
+    if (!sync_grid(S, arrivals, A.polls)) return false;
   }
   // ---- the gradient, a warp an angle
   for (int e = static_cast<int>(cta * G::warps) + warp; e < L * n * 2; e += static_cast<int>(ctas) * G::warps) {
@@ -449,16 +463,13 @@ template <int n>
 __global__ void __launch_bounds__(256, 1) grid_circuit_kernel(const __grid_constant__ ClusterArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   if (run_grid<n>(A, smem)) return;
-  if (threadIdx.x == 0) atomicMax(A.counter, kGridLost);
+  if (threadIdx.x == 0)
+    *static_cast<volatile unsigned *>(&grid_state(A, n)->lost) = 1u;
   const double nan = __longlong_as_double(0x7ff8000000000000ll);  // a CTA did not arrive
   if (A.energy_out && blockIdx.x == 0 && threadIdx.x == 0) A.energy_out[A.item.index] = nan;
   if (A.grad_out)
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 2 * n * A.item.L; e += gridDim.x * blockDim.x)
       A.grad_out[A.item.param_off + e] = nan;
-}
-
-size_t grid_doubles(int max_layers) {  // behind the vectors, without the state
-  return static_cast<size_t>(max_layers) * kGridRec * kMostGridCtas + kMostGridCtas;
 }
 
 template <int n>
@@ -487,9 +498,10 @@ struct GridShape {
     int count = 0;
     cudaError_t e = ctas(A.max_layers, &count);
     if (e != cudaSuccess) return e;
-    if (count < 1 || A.count != 1 || A.items != nullptr || A.counter == nullptr) return cudaErrorInvalidValue;
-    void *state = reinterpret_cast<double *>(A.memory + (size_t{4} << n)) + grid_doubles(A.max_layers);
-    if ((e = cudaMemsetAsync(state, 0, sizeof(GridState), s)) != cudaSuccess) return e;
+    if (count < 1 || A.count != 1 || A.items != nullptr) return cudaErrorInvalidValue;
+    // (a backward that resumes a forward leaves what that one lost)
+    const size_t bytes = A.resume ? sizeof(unsigned) : sizeof(GridState);
+    if ((e = cudaMemsetAsync(grid_state(A, n), 0, bytes, s)) != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at;
     cfg.gridDim = dim3(static_cast<unsigned>(count));
@@ -516,6 +528,8 @@ bool with_grid(int n, F &&f) {
 }
 
 }  // namespace
+
+const unsigned *grid_lost_flag(const ClusterArgs &A) { return &grid_state(A, A.n)->lost; }
 
 size_t grid_memory_values(int n, int max_layers) {
   return (size_t{4} << n) + grid_doubles(max_layers) / 2 + 1 + sizeof(GridState) / sizeof(double2) + 1;

@@ -270,6 +270,13 @@ rsv_status rsv_analytic_layers(rsv_backend *backend, int *max_layers_out, int *u
 rsv_status rsv_set_kernels(rsv_backend *backend, int flags);
 rsv_status rsv_kernels(rsv_backend *backend, int *flags_out, int *tma_passes_out);
 
+/* How often a block of a whole-device call (one circuit of 17 to 20 qubits)
+ * looks at a barrier whether the others have arrived, before it gives up for all
+ * of them (default: about a second's worth; 0 gives up at once).  The call's
+ * energy and whole gradient are NaN then, and the synchronous entry points
+ * return RSV_ERR_CUDA; later calls are not affected.  No reference counterpart. */
+rsv_status rsv_set_barrier_polls(rsv_backend *backend, int polls);
+
 /*
  * Autotuner.  Times every plan candidate of the backend's circuit -- backward
  * schedule (checkpoint where its buffers fit, uncompute), three or two
