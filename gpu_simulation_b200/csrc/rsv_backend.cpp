@@ -836,6 +836,11 @@ struct DevBuf {
     count = 0;
     owned = true;
   }
+  void swap(DevBuf &o) {
+    std::swap(p, o.p);
+    std::swap(count, o.count);
+    std::swap(owned, o.owned);
+  }
   ~DevBuf() { release(); }
 };
 
@@ -872,7 +877,9 @@ struct rsv_backend {
   int device = 0, sms = 0;
   cudaStream_t stream = nullptr;
   rsv::Plan plan;
-  rsv::DevBuf<double2> states;  // plan.num_bufs state buffers of state_len amplitudes each
+  // tile passes: plan.num_bufs state buffers of state_len amplitudes each; ring: the
+  // kept components; cluster: its memory, psi and H psi of a split call
+  rsv::DevBuf<double2> states;
   int backward_mode = RSV_BACKWARD_AUTO;
   // RSV_KERNELS_* flags (rsv_set_kernels): TMA-fed backward passes where
   // eligible, the field terms on the tile of the last layer's first backward
@@ -910,7 +917,7 @@ struct rsv_backend {
   rsv::DevBuf<double2> mps_tsite, mps_btab, mps_coslo, mps_coshi, mps_mtab, mps_wtab, mps_zt, mps_ylo, mps_yhi, mps_partials,
       mps_gf;
   // what runs a call: the tile passes, the contraction along the ring
-  // (rsv_ring.cu; its kept components lie in the state buffers) or the
+  // (rsv_ring.cu) or the
   // cluster-resident state (rsv_cluster.cu, rsv_tiles.cu, rsv_grid.cu); and the
   // field of the last forward
   rsv::Path path = rsv::Path::kPasses;
@@ -2201,7 +2208,7 @@ void assign_backward_kernels(rsv_backend *B) {
     s.kernel = kKernelDefault;
     if (!(B->kernel_flags & RSV_KERNELS_TMA)) continue;
     fill_pass_params(B, s, P);
-    if (!make_tma_pass(P, B->pipeline_err.p, B->tma[i], nullptr)) continue;
+    if (!make_tma_pass(P, B->pipeline_err.p, B->tma[i], B->path == Path::kPasses, nullptr)) continue;
     s.kernel = kKernelTma;
     s.grid = static_cast<int>(std::min<u64>(s.tile.num_tiles, static_cast<u64>(bwd_tma_blocks_per_sm(B->tma[i].kind)) *
                                                                    static_cast<u64>(std::max(1, B->sms))));
@@ -2211,45 +2218,49 @@ void assign_backward_kernels(rsv_backend *B) {
   assign_energy_fusion(B);
 }
 
+// What the ring or the cluster path keeps in B->states.
+size_t direct_values(const rsv_backend *B) {
+  if (B->path == Path::kRing)
+    return 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs;
+  return cluster_memory_values(B->n, B->cluster_shape, B->L) + 2 * B->state_len;
+}
+
 // (Re)plan a backend for a backward schedule and allocate what depends on the
 // plan: the state buffers, the product tables, the partial records and the
-// plan tables.  A failed allocation of the checkpoint schedule falls back to
+// plan tables.  The ring and cluster paths allocate their own few MB instead of
+// the tile passes' buffers, which another choice of path re-plans for.  A failed
+// allocation of the checkpoint schedule falls back to
 // the three-buffer schedule when the mode is automatic.
 void setup_plan(rsv_backend *B, int mode) {
   if (mode != RSV_BACKWARD_AUTO && mode != RSV_BACKWARD_UNCOMPUTE && mode != RSV_BACKWARD_CHECKPOINT)
     invalid("backward mode must be RSV_BACKWARD_AUTO, _UNCOMPUTE or _CHECKPOINT");
   const bool want = mode == RSV_BACKWARD_CHECKPOINT ||
                     (mode == RSV_BACKWARD_AUTO && checkpoint_fits(B->n, B->L, B->analytic_layers, B->force_c));
+  ++B->generation;  // any state kept for a deferred backward is gone
+  B->forward_only_state = false;
   B->states.release();
   Plan pl = make_plan(B->n, B->L, B->sms, want, B->analytic_layers, B->force_c);
   B->state_len = size_t{1} << pl.phys;
   B->path = choose_path(B, mode);
-  size_t values = 0;
-  if (B->path == Path::kRing)
-    values = 2 * ring_component_values(B->n, B->L) + static_cast<size_t>(B->n) * 4 * kRingDerivs;
-  else if (B->path == Path::kCluster)
-    values = cluster_memory_values(B->n, B->cluster_shape, B->L) + 2 * B->state_len;
-  if (values > static_cast<size_t>(pl.num_bufs) * B->state_len) {
+  if (B->path != Path::kPasses) {
     try {
-      B->states.alloc(values);
+      B->states.alloc(direct_values(B));
     } catch (const Error &e) {
       if (e.status != RSV_ERR_OUT_OF_MEMORY) throw;
-      cudaGetLastError();  // clear the allocation failure
       B->path = Path::kPasses;
     }
   }
-  if (B->states.p == nullptr) try {
-    B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
-  } catch (const Error &e) {
-    if (mode != RSV_BACKWARD_AUTO || !pl.checkpoint || e.status != RSV_ERR_OUT_OF_MEMORY) throw;
-    cudaGetLastError();  // clear the allocation failure
-    pl = make_plan(B->n, B->L, B->sms, false, B->analytic_layers, B->force_c);
-    B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
+  if (B->path == Path::kPasses) {
+    try {
+      B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
+    } catch (const Error &e) {
+      if (mode != RSV_BACKWARD_AUTO || !pl.checkpoint || e.status != RSV_ERR_OUT_OF_MEMORY) throw;
+      pl = make_plan(B->n, B->L, B->sms, false, B->analytic_layers, B->force_c);
+      B->states.alloc(static_cast<size_t>(pl.num_bufs) * B->state_len);
+    }
+    // (zero padding for n < 12)
+    check(cudaMemset(B->states.p, 0, B->states.count * sizeof(double2)), "state memset");
   }
-  // (zero padding for n < 12; the other paths need none)
-  check(cudaMemset(B->states.p, 0, std::min(B->states.count, static_cast<size_t>(pl.num_bufs) * B->state_len) *
-                                       sizeof(double2)),
-        "state memset");
   B->plan = pl;
   B->backward_mode = mode;
   B->num_bwd_passes = static_cast<int>(B->plan.bwd.size());
@@ -2285,8 +2296,6 @@ void setup_plan(rsv_backend *B, int mode) {
   B->order.alloc(ord.size());
   check(cudaMemcpy(B->order.p, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice),
         "order upload");
-  ++B->generation;  // any state kept for a deferred backward is gone
-  B->forward_only_state = false;
 }
 
 // ------------------------------------------------------------------------
@@ -2674,6 +2683,21 @@ rsv_status rsv_benchmark_forward_graph(rsv_backend *B, const double *params, siz
     if (repeats == 0) invalid("repeats must be at least 1.");
     if (normal_ms_out == nullptr || graph_ms_out == nullptr) invalid("output pointer is null");
     cudaStream_t st = B->stream;
+    // the tile passes' buffers, for this call, where the engine runs another path
+    struct Lent {
+      DevBuf<double2> &states, passes;
+      bool lent = false;
+      explicit Lent(DevBuf<double2> &s) : states(s) {}
+      ~Lent() {
+        if (lent) states.swap(passes);
+      }
+    } buffers(B->states);
+    if (B->path != Path::kPasses) {
+      buffers.passes.alloc(static_cast<size_t>(B->plan.num_bufs) * B->state_len);
+      check(cudaMemsetAsync(buffers.passes.p, 0, buffers.passes.count * sizeof(double2), st), "state memset");
+      buffers.states.swap(buffers.passes);
+      buffers.lent = true;
+    }
     ++B->generation;
     B->forward_only_state = false;
     upload_host_coefs(B, params, st);

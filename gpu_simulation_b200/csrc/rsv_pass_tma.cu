@@ -984,16 +984,16 @@ bool tma_pass_shape_ok(const PassParams &P, std::string *why) {
   return map_dims(P, ld, st, why);
 }
 
-bool make_tma_pass(const PassParams &P, int *err, TmaPass &out, std::string *why) {
+bool make_tma_pass(const PassParams &P, int *err, TmaPass &out, bool maps, std::string *why) {
   if (!tma_pass_shape_ok(P, why)) return false;
   std::vector<MapDim> ld, st;
   if (!map_dims(P, ld, st, why)) return false;
   std::memset(&out, 0, sizeof(out));
   int sh[kTmaRank];
   unsigned mk[kTmaRank];
-  if (!encode(out.psi_map, P.psi_in, P.n, ld, out.ld_shift, out.ld_mask, why)) return false;
-  if (!encode(out.lam_map, P.lam_in, P.n, ld, sh, mk, why)) return false;
-  if (P.tile_bits == 11 && !encode(out.out_map, P.lam_out, P.n, st, out.st_shift, out.st_mask, why)) return false;
+  if (maps && !encode(out.psi_map, P.psi_in, P.n, ld, out.ld_shift, out.ld_mask, why)) return false;
+  if (maps && !encode(out.lam_map, P.lam_in, P.n, ld, sh, mk, why)) return false;
+  if (maps && P.tile_bits == 11 && !encode(out.out_map, P.lam_out, P.n, st, out.st_shift, out.st_mask, why)) return false;
   out.err = err;
   out.kind = P.tile_bits == 12 ? kTmaLow : kTmaHalf;
   return true;

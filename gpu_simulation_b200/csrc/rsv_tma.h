@@ -82,7 +82,8 @@ bool tma_pass_shape_ok(const PassParams &P, std::string *why);
 // Encodes the three tensor maps of the pass (needs a CUDA context on the
 // device that owns the buffers).  Returns false (with the reason) when the
 // pass is not eligible or the driver rejects a map; nothing is allocated.
-bool make_tma_pass(const PassParams &P, int *err, TmaPass &out, std::string *why);
+// Without `maps` only the eligibility by shape (a plan whose buffers do not exist).
+bool make_tma_pass(const PassParams &P, int *err, TmaPass &out, bool maps, std::string *why);
 
 // The tile bits in the order the TMA kernels rotate them (undo order).
 constexpr int kTmaRotationOrder[8] = {7, 8, 9, 10, 3, 4, 5, 6};

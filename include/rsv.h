@@ -75,7 +75,9 @@ const char *rsv_stage_name(int i);
  * every engine.  structured_rotation_chunk_width must be in
  * [1, 8] and double_buffer is accepted; both are validated as the reference
  * does and otherwise ignored (the engine plans its own tiles).
- * Allocates three state buffers of 16 * 2^max(n,12) bytes.
+ * The tile passes need two, three or more state buffers of 16 * 2^max(n,12)
+ * bytes (rsv_backward_mode).  The two paths below allocate a few MB instead;
+ * choosing the tile passes for such an engine later allocates their buffers then.
  * A structured_adjoint circuit of few layers is contracted along the ring
  * (gpu_simulation_b200/csrc/rsv_ring.cu), another one of up to 16 qubits and
  * 64 layers keeps its state in one thread-block cluster (rsv_cluster.cu),
