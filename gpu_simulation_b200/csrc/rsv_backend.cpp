@@ -1374,11 +1374,17 @@ void run_gate_level(rsv_backend *B, bool grad, double *energy_out, double *grad_
   check(rsv::run_gate_level(A, st), "gate-level launch");
 }
 
+void check_planned(const rsv_backend *B) {
+  if (B->states.p == nullptr)
+    throw Error(RSV_ERR_OUT_OF_MEMORY, "the backend's state buffers could not be allocated; choose a schedule that fits");
+}
+
 // d_params: the angles on the device, or null when B->coef holds their cosines
 // and sines.  keep: an energy-only call whose gradient may be asked for later
 // (rsv_backward_device).
 void run_all(rsv_backend *B, const double *d_params, bool grad, double *energy_out, double *grad_out,
              cudaStream_t st, bool keep = false) {
+  check_planned(B);
   ++B->generation;
   B->forward_only_state = false;
   if (B->path != Path::kPasses) {
@@ -2230,10 +2236,22 @@ size_t direct_values(const rsv_backend *B) {
 // plan tables.  The ring and cluster paths allocate their own few MB instead of
 // the tile passes' buffers, which another choice of path re-plans for.  A failed
 // allocation of the checkpoint schedule falls back to
-// the three-buffer schedule when the mode is automatic.
+// the three-buffer schedule when the mode is automatic.  Where it throws, the
+// backend has no state buffers and refuses calls (check_planned) until a re-plan
+// succeeds.
+void plan_and_allocate(rsv_backend *B, int mode);
 void setup_plan(rsv_backend *B, int mode) {
   if (mode != RSV_BACKWARD_AUTO && mode != RSV_BACKWARD_UNCOMPUTE && mode != RSV_BACKWARD_CHECKPOINT)
     invalid("backward mode must be RSV_BACKWARD_AUTO, _UNCOMPUTE or _CHECKPOINT");
+  try {
+    plan_and_allocate(B, mode);
+  } catch (...) {
+    B->states.release();
+    throw;
+  }
+}
+
+void plan_and_allocate(rsv_backend *B, int mode) {
   const bool want = mode == RSV_BACKWARD_CHECKPOINT ||
                     (mode == RSV_BACKWARD_AUTO && checkpoint_fits(B->n, B->L, B->analytic_layers, B->force_c));
   ++B->generation;  // any state kept for a deferred backward is gone
@@ -2599,6 +2617,7 @@ rsv_status rsv_profile_energy_and_grad(rsv_backend *B, const double *params, siz
     validate_params(B, params, num_params);
     if (energy_out == nullptr || stage_ms_out == nullptr) invalid("output pointer is null");
     if (compute_gradient && gradient_out == nullptr) invalid("gradient_out is null");
+    check_planned(B);
     cudaStream_t st = B->stream;
     cudaEvent_t ev[8];
     for (auto &e : ev) check(cudaEventCreate(&e), "cudaEventCreate");
@@ -2682,6 +2701,7 @@ rsv_status rsv_benchmark_forward_graph(rsv_backend *B, const double *params, siz
     validate_params(B, params, num_params);
     if (repeats == 0) invalid("repeats must be at least 1.");
     if (normal_ms_out == nullptr || graph_ms_out == nullptr) invalid("output pointer is null");
+    check_planned(B);
     cudaStream_t st = B->stream;
     // the tile passes' buffers, for this call, where the engine runs another path
     struct Lent {

@@ -72,3 +72,33 @@ def test_a_ring_circuit_runs_on_an_almost_full_device():
     del full
     torch.cuda.empty_cache()
     assert e == e_ref and np.array_equal(g, g_ref)
+
+
+def test_a_schedule_that_does_not_fit_is_refused_and_so_are_calls_until_one_does():
+    """28 qubits, 40 layers: the checkpoints (two buffers of 4 GiB a layer) are
+    more than any device's memory."""
+    import torch
+
+    from gpu_simulation_b200._lib import EngineError, check
+
+    n, layers = 28, 40
+    p = np.random.default_rng(4).uniform(0.0, 2.0 * np.pi, 2 * n * layers)
+    eng = Engine(n, layers, 1.0)
+    x = torch.tensor(p, device="cuda", requires_grad=True)
+    v = ring_ising_energy(x, eng)
+    with pytest.raises(EngineError):
+        eng.set_backward_mode("checkpoint")
+    d, e, g = x.detach(), torch.zeros(1, dtype=torch.float64, device="cuda"), torch.zeros_like(x.detach())
+    for call in (lambda: eng.energy(p), lambda: eng.energy_and_grad(p), lambda: eng.energy_and_grad_device(d, e, g),
+                 lambda: eng.profile_energy_and_grad(p), lambda: eng.benchmark_forward_graph(p, repeats=1),
+                 lambda: ring_ising_energy(x, eng), v.backward):
+        with pytest.raises(EngineError):
+            call()
+    assert not g.any()
+    assert eng.device_bytes() < 1 << 30
+    eng.set_backward_mode("auto")
+    assert abs(eng.energy(p) - v.item()) < 1e-12
+    with pytest.raises(ValueError):
+        check(eng._lib.rsv_set_backward_mode(eng._h, 9))
+    assert abs(eng.energy(p) - v.item()) < 1e-12  # an unknown mode changes nothing
+    eng.close()
