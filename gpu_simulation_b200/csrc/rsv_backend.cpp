@@ -3063,7 +3063,9 @@ rsv_status rsv_batch_info(rsv_batch *batch, int *count, size_t *num_params, int 
     if (count) *count = batch->count;
     if (num_params) *num_params = batch->num_params;
     if (slots) *slots = batch->active_slots;
-    if (device_bytes) *device_bytes = batch->slot_bytes * static_cast<size_t>(batch->slots);
+    if (device_bytes)
+      *device_bytes = batch->slot_bytes * static_cast<size_t>(batch->slots) + batch->d_vectors.count * sizeof(double2) +
+                      batch->d_items.count * sizeof(ClusterItem) + batch->d_counters.count * sizeof(int);
   });
 }
 

@@ -381,7 +381,8 @@ rsv_status rsv_batch_destroy(rsv_batch *batch);
 rsv_status rsv_batch_set_circuits(rsv_batch *batch, int count, const int *num_qubits,
                                   const int *num_layers, const double *fields);
 
-/* Circuits and packed parameter count of the current description. */
+/* Circuits and packed parameter count of the current description; device_bytes:
+ * the persistent kernel's scratch and what the resident circuits hold beside it. */
 rsv_status rsv_batch_info(rsv_batch *batch, int *count, size_t *num_params, int *slots,
                           size_t *device_bytes);
 

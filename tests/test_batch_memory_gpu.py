@@ -98,3 +98,15 @@ def test_a_description_that_failed_is_not_run():
     eng.run_device(d, e, g)
     assert np.array_equal(g.cpu().numpy(), g_ref)
     eng.close()
+
+
+def test_reported_bytes_hold_the_resident_circuits_vectors():
+    eng = BatchEngine()
+    before = eng.device_bytes()
+    eng.set_circuits([12] * 4, [2] * 4, [1.0] * 4)
+    in_registers = eng.device_bytes()
+    eng.set_circuits([16] * 4, [2] * 4, [1.0] * 4)
+    tiled = eng.device_bytes()
+    eng.close()
+    assert before < in_registers < before + (1 << 16)  # descriptors alone
+    assert tiled >= in_registers + 4 * (4 << 20)  # psi and lambda, two of each, of 2^16 amplitudes
