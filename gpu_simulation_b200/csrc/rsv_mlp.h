@@ -25,8 +25,9 @@ struct MlpGemm {
 };
 // One or two independent products in one launch.
 cudaError_t mlp_gemm(const MlpGemm *g, int count, cudaStream_t s);
-cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout, float *loss,
-                    cudaStream_t s);
+// partials: 256 floats
+cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout, float *partials,
+                    float *loss, cudaStream_t s);
 cudaError_t gd_step(long long count, double *p, const double *g, double stepsize, const double *energy,
                     double *energy_hist, double *gnorm_hist, int *counter, cudaStream_t s);
 cudaError_t adam_vqe_step(long long count, double *p, const double *g, double *m, double *v, double lr,

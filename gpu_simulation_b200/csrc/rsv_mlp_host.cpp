@@ -198,7 +198,7 @@ rsv_status rsv_mlp_mse(size_t count, const float *d_out, const float *d_target, 
   return mlp_guarded([&] {
     if (count == 0) throw ArgError("count must be positive");
     if (!d_out || !d_target || !d_dout || !d_loss || !d_partials) throw ArgError("null device pointer");
-    cuda_check(mlp_mse(static_cast<long long>(count), d_out, d_target, d_dout, d_loss,
+    cuda_check(mlp_mse(static_cast<long long>(count), d_out, d_target, d_dout, d_partials, d_loss,
                        static_cast<cudaStream_t>(stream)),
                "mse");
   });
