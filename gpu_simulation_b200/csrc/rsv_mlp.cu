@@ -44,6 +44,17 @@ constexpr int kGemmThreads = kGroups * kGroupThreads;
 // us by this limit: none shared 79, 160 75.7, 296 76.9, 400 to 444 70.7, 592 78.6, 900 85.4; on
 // 32 rows 50 without and 41 with, on 1024 rows 125 and 109.
 constexpr int kMostBlocks = 444;
+// A product of small depth and many tiles has nothing to gain from a split depth, and
+// pays for its idle groups and their meeting: from kWholeTiles tiles on, one that is
+// less than 128 deep gives every group a tile of its own.  Us, split and whole
+// (64 x 64 tiles took): 3 -> 64 on 16384 rows (1024 tiles) 14.6 and 11.3 (16), on
+// 131072 82 and 17 (18); 3 -> 256 on 131072 320 and 58 (60); 32 -> 256 336 and 123
+// (202); 64 -> 256 407 and 224 (386); 96 -> 64 158 and 87 (146); with 512 tiles
+// and less the two are equal within 5 %, and the split sum is the more exact one.
+// 128 deep and more the split form is the faster one against the 64 x 64 tiles too
+// (128 -> 256 636, 754) and stays.  kWholeCtas: resident CTAs that the registers are
+// limited for (3 -> 256 on 131072 rows: 2 74, 3 61, 4 58, 5 70).
+constexpr int kWholeDepth = 127, kWholeTiles = 1024, kWholeCtas = 4;
 constexpr int kPad = kTile + 4;    // 16-byte rows, two-way conflicts at most on the stores
 
 __device__ __forceinline__ float gelu(float z) {
@@ -63,24 +74,29 @@ struct GemmPair {
   int log_splits[2], blocks[2];  // log2 of the CTAs (a cluster) that share a tile's depth; all, in whole clusters
 };
 
-template <bool shared_depth>
-__global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constant__ GemmPair P) {
+// How the four groups of a CTA work: on one tile, each with a part of its depth
+// (the CTA's, or its cluster's share of it); or each on a tile of its own.
+enum class Depth { kSplit, kShared, kWhole };
+
+template <Depth form>
+__global__ void __launch_bounds__(kGemmThreads, form == Depth::kWhole ? kWholeCtas : 0) gemm_kernel(const __grid_constant__ GemmPair P) {
+  constexpr bool shared_depth = form == Depth::kShared, whole = form == Depth::kWhole;
   __shared__ float stage[kGroups][2][2][kTileK][kPad];  // [group][buffer][A, B][k][m or n]
   __shared__ float rows[kGroups][kTile];
   const int which = static_cast<int>(blockIdx.x) < P.blocks[0] ? 0 : 1;
   const MlpGemm &g = P.g[which];
   const int log_splits = shared_depth ? P.log_splits[which] : 0, splits = 1 << log_splits;
   const int block = static_cast<int>(blockIdx.x) - (which ? P.blocks[0] : 0);
-  const int tile = block >> log_splits, share = block & (splits - 1);
-  if (tile >= P.tiles[which]) return;  // fills up the last cluster
-  const int m0 = tile / P.tiles_n[which] * kTile, n0 = tile % P.tiles_n[which] * kTile;
   const int tid = threadIdx.x, group = tid / kGroupThreads, t = tid % kGroupThreads;
+  const int tile = whole ? block * kGroups + group : block >> log_splits, share = block & (splits - 1);
+  if (tile >= P.tiles[which]) return;  // fills up the last cluster, or the last CTA's groups
+  const int m0 = tile / P.tiles_n[which] * kTile, n0 = tile % P.tiles_n[which] * kTile;
   const int tx = t % 8, ty = t / 8;
   const int M = g.M, N = g.N, K = g.K;
   // this group's depth range, whole stages
   const int parts = kGroups * splits;
   const int span = ((K + parts * kTileK - 1) >> (log_splits + 6)) * kTileK;  // 64 = kGroups * kTileK
-  const int first = (share * kGroups + group) * span, end = first + span < K ? first + span : K;
+  const int first = whole ? 0 : (share * kGroups + group) * span, end = whole || first + span >= K ? K : first + span;
   // threads run along the contiguous index of each operand
   const bool ak = g.sak == 1, bk = g.sbk == 1;
   const int a_m = ak ? t / 16 : t % 32, a_k = ak ? t % 16 : t / 32, a_dm = ak ? 4 : 0, a_dk = ak ? 0 : 2;
@@ -113,6 +129,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
     if (k0 + kTileK < end) load(k0 + kTileK);
 #pragma unroll
     for (int kk = 0; kk < kTileK; ++kk) {
+      if (whole && kk % 4 == 0 && k0 + kk >= K) break;  // (a depth of 3 is common)
       const float4 a = *reinterpret_cast<const float4 *>(&As[kk][4 * ty]);
       const float4 c = *reinterpret_cast<const float4 *>(&Bs[kk][4 * tx]);
       const float av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
@@ -125,16 +142,6 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
 #pragma unroll
       for (int kk = 0; kk < kTileK; ++kk) row += As[kk][t];
   }
-  // the groups' parts, added in group order
-  __syncthreads();
-  float *part = &stage[0][0][0][0][0];  // [group][kTile][kTile + 1]
-  constexpr int kRow = kTile + 1, kPart = kTile * kRow;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) part[group * kPart + (4 * ty + i) * kRow + 4 * tx + j] = acc[i][j];
-  if (sums) rows[group][t] = row;
-  __syncthreads();
   auto finish = [&](int i, int j, float z) {
     const int m = m0 + i, n = n0 + j;
     if (m >= M || n >= N) return;
@@ -145,6 +152,47 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
     if (g.gelu_of != nullptr) z *= gelu_grad(g.gelu_of[at]);
     g.C[at] = z;
   };
+  if constexpr (whole) {  // straight from the registers: a warp's 16-byte stores are whole lines
+    const int n = n0 + 4 * tx;
+    const bool vec = N % 4 == 0 && ((reinterpret_cast<size_t>(g.C) | reinterpret_cast<size_t>(g.Z)) & 15) == 0;
+    float b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = g.bias != nullptr && n + j < N ? g.bias[n + j] : -0.0f;  // (x + -0 is x)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + 4 * ty + i;
+      if (m >= M || n >= N) return;
+      const long long at = static_cast<long long>(m) * N + n;
+      float z[4], c[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        z[j] = acc[i][j] + b[j];
+        c[j] = g.gelu ? gelu(z[j]) : z[j];
+      }
+      if (vec) {
+        if (g.Z != nullptr) *reinterpret_cast<float4 *>(g.Z + at) = make_float4(z[0], z[1], z[2], z[3]);
+        *reinterpret_cast<float4 *>(g.C + at) = make_float4(c[0], c[1], c[2], c[3]);
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (n + j >= N) break;
+        if (g.Z != nullptr) g.Z[at + j] = z[j];
+        g.C[at + j] = c[j];
+      }
+    }
+    return;
+  }
+  // the groups' parts, added in group order
+  __syncthreads();
+  float *part = &stage[0][0][0][0][0];  // [group][kTile][kTile + 1]
+  constexpr int kRow = kTile + 1, kPart = kTile * kRow;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) part[group * kPart + (4 * ty + i) * kRow + 4 * tx + j] = acc[i][j];
+  if (sums) rows[group][t] = row;
+  __syncthreads();
 #pragma unroll
   for (int e = tid; e < kTile * kTile; e += kGemmThreads) {
     const int i = e / kTile, j = e % kTile;
@@ -305,6 +353,12 @@ cudaError_t mlp_gemm(const MlpGemm *g, int count, cudaStream_t s) {
     P.tiles_n[k] = (g[k].N + kTile - 1) / kTile;
     P.tiles[k] = P.tiles_n[k] * ((g[k].M + kTile - 1) / kTile);
   }
+  if (count == 1 && g[0].row_sums == nullptr && g[0].gelu_of == nullptr && g[0].K <= kWholeDepth &&
+      P.tiles[0] >= kWholeTiles) {
+    P.blocks[0] = (P.tiles[0] + kGroups - 1) / kGroups;
+    gemm_kernel<Depth::kWhole><<<P.blocks[0], kGemmThreads, 0, s>>>(P);
+    return cudaGetLastError();
+  }
   // as many CTAs a tile as give every group a stage and keep the launch within kMostBlocks
   int size = 1;
   auto plan = [&](int most) {
@@ -330,7 +384,8 @@ cudaError_t mlp_gemm(const MlpGemm *g, int count, cudaStream_t s) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = size > 1 ? 1 : 0;
-  return size > 1 ? cudaLaunchKernelEx(&cfg, gemm_kernel<true>, P) : cudaLaunchKernelEx(&cfg, gemm_kernel<false>, P);
+  return size > 1 ? cudaLaunchKernelEx(&cfg, gemm_kernel<Depth::kShared>, P)
+                  : cudaLaunchKernelEx(&cfg, gemm_kernel<Depth::kSplit>, P);
 }
 
 cudaError_t mlp_mse(long long count, const float *out, const float *target, float *dout, float *partials,
