@@ -527,12 +527,6 @@ bool with_shape(int n, ClusterShape h, F &&f) {
 
 }  // namespace
 
-bool cluster_shape_built(int n, ClusterShape h) {
-  if (n > kClusterMaxQubits) return h.tiled && n <= kGridMaxQubits;
-  if (h.tiled) return tile_shape_built(n, h);
-  return with_shape(n, h, [](auto) {});
-}
-
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s) {
   if (A.count < 1) return cudaSuccess;
   if (A.n > kClusterMaxQubits) return launch_grid(A, s);

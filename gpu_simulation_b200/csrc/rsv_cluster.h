@@ -53,7 +53,6 @@ struct ClusterArgs {
 // Polls of a whole-device barrier: about a second.
 constexpr int kGridPolls = 1 << 21;
 
-bool cluster_shape_built(int n, ClusterShape h);
 // Global memory of a cluster: psi's checkpoints, or a tiled circuit's vectors.
 size_t cluster_memory_values(int n, ClusterShape h, int max_layers);
 cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s);
@@ -61,7 +60,6 @@ cudaError_t launch_cluster(const ClusterArgs &A, cudaStream_t s);
 cudaError_t cluster_capacity(int n, ClusterShape h, int max_layers, int *clusters);
 
 // Tiled circuits (rsv_tiles.cu); the functions above go there.
-bool tile_shape_built(int n, ClusterShape h);
 cudaError_t launch_tiles(const ClusterArgs &A, cudaStream_t s);
 cudaError_t tile_capacity(int n, ClusterShape h, int max_layers, int *clusters);
 

@@ -564,10 +564,6 @@ bool with_tiles(int n, int log_ctas, F &&f) {
 
 }  // namespace
 
-bool tile_shape_built(int n, ClusterShape h) {
-  return with_tiles(n, h.log_ctas, [](auto) {});
-}
-
 cudaError_t launch_tiles(const ClusterArgs &A, cudaStream_t s) {
   cudaError_t e = cudaErrorInvalidValue;
   with_tiles(A.n, A.shape.log_ctas, [&](auto shape) {

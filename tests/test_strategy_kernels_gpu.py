@@ -39,6 +39,7 @@ def test_strategy_keeps_its_kernels(strategy, name, n, layers):
         x.grad = None
         v = ring_ising_energy(x, eng)
         if interrupted:
+            torch.cuda.synchronize()  # the host call runs on the engine's own stream
             eng.energy(p[::-1].copy())
         v.backward()
         assert abs(v.item() - e_ref) < TOL
