@@ -2160,8 +2160,8 @@ void assign_energy_fusion(rsv_backend *B) {
 // faster one below 12 qubits (L = 4, energy and gradient: n = 10 18 us against
 // 25, n = 12 37 against 27), and the tile passes never are (n = 12 142 us, n =
 // 28 21 400 against 38).  5 layers are faster on the ring from 20 qubits on (216
-// us against about 270; n = 16 178 against 125 tiled, n = 17 182 against 146, n = 19
-// 212 against 158; the energy alone 46 against 43, 49 against 57, 53 against 60).
+// us against about 260; n = 16 178 against 125 tiled, n = 17 182 against 139, n = 19
+// 212 against 157; the energy alone 46 against 43, 49 against 53, 53 against 57).
 bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 20 && L == 5); }
 
 // How a single circuit is spread over a cluster (rsv_cluster.cu), the fastest of
@@ -2174,8 +2174,8 @@ bool ring_rule(int n, int L) { return (n >= 12 && L <= 4) || (n >= 20 && L == 5)
 // 64), and with 16 qubits the exchanges cost more than passing the state through
 // memory, tiled (184 us against 258; 15 qubits 167 against 163, 14 qubits 167
 // against 123).  From 17 qubits on that takes the whole device: L = 6 and 16, us,
-// against the tile passes: n = 17 173 and 453 (226, 740), n = 18 176 and 452 (228,
-// 744), n = 19 185 and 481 (236, 784), n = 20 319 and 822 (337, 1115).
+// against the tile passes: n = 17 165 and 434 (226, 740), n = 18 168 and 432 (228,
+// 744), n = 19 185 and 479 (236, 784), n = 20 314 and 815 (337, 1115).
 ClusterShape cluster_shape_for(int n) {
   if (n <= 9) return {0, 2, false};
   if (n <= 11) return {0, 3, false};

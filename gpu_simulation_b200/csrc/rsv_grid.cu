@@ -11,12 +11,13 @@
 //
 // Before, every pass was a launch of the general tile-pass kernels (two passes a
 // layer and direction, 20 qubits: forward 12 to 13.5 us, backward 25 to 31),
-// with the first three layers as matrix products.  A layer now takes 28 us from
-// 17 to 19 qubits, a tile or less a CTA, of which the four barriers are about 8;
-// with 20 qubits 50 us: 108 of 148 CTAs have a second tile, which the others wait
-// for (issuing its loads ahead, as rsv_tiles.cu does, made L = 8 456 us instead of
-// 422).  Energy and gradient at L = 8: n = 17 330 -> 230 us, n = 18 331 -> 229, n =
-// 19 349 -> 246, n = 20 493 -> 422.
+// with the first three layers as matrix products.  A layer now takes 27 to 29 us from
+// 17 to 19 qubits, a tile or less a CTA, and 50 us with 20 qubits: 108 of 148 CTAs
+// have a second tile, which the others wait for (issuing its loads ahead, as
+// rsv_tiles.cu does, made L = 8 456 us instead of the 422 of that time).  More warps
+// wait at a barrier than for anything else (n = 20: 3.7 for each that issues; next are
+// loads with 2.3); FP64 and L2 are each busy a fifth of the time.  Energy and gradient
+// at L = 8: n = 17 330 -> 219 us, n = 18 331 -> 220, n = 19 349 -> 245, n = 20 493 -> 415.
 #include <cuda_runtime.h>
 
 #include <atomic>

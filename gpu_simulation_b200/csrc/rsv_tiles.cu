@@ -21,10 +21,11 @@
 // uses the exchange buffers, a low pass a third one for psi, where the tables of
 // a deep circuit leave room).
 //
-// What bounds it: FP64 (about 5 us a tile and layer), the loads and stores from
-// L2 (6 us) and the exchanges (3 us) follow each other more than they overlap,
-// since two vectors of 16 amplitudes leave a SM 8 warps: 15 to 18 us a tile and
-// layer.  Keeping the state in registers instead costs 25 (n = 13) to 47 us (n =
+// What bounds it: FP64, the loads and stores from L2 and the exchanges follow each
+// other more than they overlap, since two vectors of 16 amplitudes leave a SM 8
+// warps: 15 to 18 us a tile and layer on one CTA a circuit.  128 circuits of n = 16,
+// L = 6 keep the FP64 pipe busy 26 % of the time, L2 30 %, L1 and shared memory 39 %,
+// and the warps wait for loads first (2.2 for each that issues).  Keeping the state in registers instead costs 25 (n = 13) to 47 us (n =
 // 16), bound by the stores into other CTAs.  148 circuits of L = 8, before
 // (registers) and now: n = 13 0.39 -> 0.26 ms, n = 14 1.13 -> 0.59, n = 15 2.61 ->
 // 1.23, n = 16 6.25 -> 2.64; 4096 mixed circuits 23.6 -> 12.2 ms; one of n = 16, L =

@@ -76,15 +76,19 @@ const char *rsv_stage_name(int i);
  * [1, 8] and double_buffer is accepted; both are validated as the reference
  * does and otherwise ignored (the engine plans its own tiles).
  * The tile passes need two, three or more state buffers of 16 * 2^max(n,12)
- * bytes (rsv_backward_mode).  The two paths below allocate a few MB instead;
- * choosing the tile passes for such an engine later allocates their buffers then.
+ * bytes (rsv_backward_mode).  The paths below allocate their own few MB instead
+ * (10 MB at n = 28, L = 4; at most 173 MB, at n = 31, L = 5); choosing the tile passes for such an engine
+ * later allocates their buffers then.
  * A structured_adjoint circuit of few layers is contracted along the ring
- * (gpu_simulation_b200/csrc/rsv_ring.cu), another one of up to 16 qubits and
- * 64 layers keeps its state in one thread-block cluster (rsv_cluster.cu),
- * instead of running the tile passes, with the same results to rounding, as
- * long as the backward schedule, the analytic layers and the kernel flags
- * below are at their defaults; setting one of them otherwise selects the tile
- * passes.
+ * (gpu_simulation_b200/csrc/rsv_ring.cu: n >= 12 and L <= 4, n >= 20 and L = 5).
+ * Another one of up to 64 layers keeps its state in the registers of one
+ * thread-block cluster up to 15 qubits (rsv_cluster.cu), passes through a
+ * cluster in tiles at 16 (rsv_tiles.cu) and through the whole device in tiles
+ * at 17 to 20 while the tables of its layers fit (rsv_grid.cu).  All in place of
+ * the tile passes, the split entry points included, and with the same results to
+ * rounding, as long as the backward schedule, the analytic layers and the kernel
+ * flags below are at their defaults; setting one of them otherwise selects the
+ * tile passes.
  */
 rsv_status rsv_create(int num_qubits, int num_layers, double field,
                       const char *gradient_strategy, int structured_rotation_chunk_width,
@@ -345,10 +349,13 @@ unsigned long long rsv_ring_map(unsigned long long index, int num_qubits, int in
  * Batched circuits: many independent ring-Ising circuits of uneven size
  * (2 <= num_qubits <= RSV_BATCH_MAX_QUBITS, 1 <= num_layers <=
  * RSV_BATCH_MAX_LAYERS, own field each) evaluated by one launch per qubit
- * count, every circuit's state resident in the registers and shared memory of
- * one thread-block cluster (the default), or by ONE persistent kernel whose
+ * count (the default): up to 12 qubits a circuit's state stays in the registers
+ * of one CTA, from 13 on it passes through 1 to 16 CTAs in tiles from memory of
+ * the handle (13 and 14 qubits in registers of 8 or 16 CTAs where few circuits
+ * leave the device idle).  Or by ONE persistent kernel whose
  * states stream through scratch slots (chosen by giving slots at creation, by
- * rsv_batch_set_active_slots or by rsv_batch_set_cluster).  No counterpart in the reference, which evaluates one circuit per
+ * rsv_batch_set_active_slots or by rsv_batch_set_cluster).  No counterpart in
+ * the reference, which evaluates one circuit per
  * backend object; a batch of circuits there is a loop over
  * RingIsingCudaBackend::energy_and_grad (reference cpp/ising_cuda_backend.hpp:38-41).
  *
