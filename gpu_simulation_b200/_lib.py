@@ -161,9 +161,12 @@ def load_library() -> ctypes.CDLL:
 def raw_stream(device_index: int) -> int:
     """The handle of torch's current stream on a device.  Without the Stream
     object that torch.cuda.current_stream builds around it (2.2 us against 0.1,
-    of a small circuit's 15 us call)."""
+    of a small circuit's 15 us call).  Like that one it refuses a tensor that is
+    on no CUDA device (index -1), which the bare handle would not."""
     import torch
 
+    if device_index < 0:
+        raise ValueError("expected a CUDA tensor")
     return torch._C._cuda_getCurrentRawStream(device_index)
 
 

@@ -42,6 +42,9 @@ class RingIsingEnergy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):
         (flat,) = ctx.saved_tensors
+        # (a saved-tensor hook may hand back another tensor than was saved)
+        if not (flat.is_cuda and flat.dtype == torch.float64 and flat.is_contiguous()):
+            raise ValueError("the saved parameters must be a contiguous float64 CUDA tensor")
         engine: Engine = ctx.engine
         grad = torch.empty_like(flat)
         status = engine._lib.rsv_backward_device(engine._h, ctx.generation, grad.data_ptr(),
